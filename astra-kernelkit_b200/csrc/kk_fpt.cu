@@ -21,6 +21,7 @@
 #include "kk_cone.cuh"
 
 #include <climits>
+#include <type_traits>
 
 namespace kk {
 
@@ -39,10 +40,30 @@ struct FptArgs {
     int slab;
     int rec0, nrec;  // records of this chunk
     int accumulate;  // add to the volume (later chunks, or additive)
-    float4* ray_ab;  // (a1, b1, a2, b2) per ray of the chunk
+    float4* ray_ab;  // per * nrec entries, laid out per record (RayRecord)
     float* ray_pc;   // projection value * corr * outputScale per ray
-    int tiled[3];    // the tile pass handles shared records along axis A
 };
+
+// Ray set-ups of one record of the chunk, by class. General records: (a1,
+// b1, a2, b2) per ray and the folded projection values, rows fastest (a warp
+// of the gather, consecutive voxels along the fastest volume axis, reads
+// neighbouring entries). Records whose rows share their D1 coordinate: per
+// ray its (a2, value) and those of the next row, as (a2, a2', value,
+// value'), columns fastest (a warp of the column pass walks consecutive
+// columns, two rays per load) and the rows in the order of v's D2
+// component, and a1 per column. b1 and b2 follow from the source.
+struct RayRecord {
+    float4* ab;
+    float* pc;  // general: the value per ray; shared: a1 per column
+};
+
+__device__ __forceinline__ RayRecord ray_record(const FptArgs& L, int k) {
+    const int64_t per = (int64_t)L.rows * L.cols;
+    RayRecord R;
+    R.ab = L.ray_ab + k * per;
+    R.pc = L.ray_pc + k * per;
+    return R;
+}
 
 constexpr int FPT_TILE_2 = 32;
 constexpr int FPT_TILE_1 = 8;
@@ -62,19 +83,27 @@ __device__ __forceinline__ float place(int k, int A, int D1, float t, float d1, 
     return k == A ? t : (k == D1 ? d1 : d2);
 }
 
-// Ray set-up of every (record, column, row) of the chunk, rows fastest: a
-// warp of the gather (consecutive voxels along the fastest volume axis,
-// which for circular scans map to consecutive detector rows) then reads
-// neighbouring entries. The projection value is folded in here, times the
-// ray's corr * outputScale.
+// circular scans: the detector's v has no component along A and D1, so
+// every row of a column has bit for bit the same D1 coordinate sequence
+// (as in the forward projector's shared path)
+__device__ __forceinline__ bool shared_record(const kk_fp_angle* P, int A, int D1) {
+    const float vA = A == 0 ? __ldg(&P->v[0]) : (A == 1 ? __ldg(&P->v[1]) : __ldg(&P->v[2]));
+    const float vD1 = D1 == 0 ? __ldg(&P->v[0]) : __ldg(&P->v[1]);
+    return vA == 0.f && vD1 == 0.f;
+}
+
+// Ray set-up of every ray of the chunk, in its record's layout. The
+// projection value is folded in here, times the ray's corr * outputScale.
 __global__ void fpt_rays_kernel(const FptArgs L) {
     const int64_t per = (int64_t)L.rows * L.cols;
     const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= per * L.nrec) return;
     const int k = (int)(id / per);
     const int cr = (int)(id - (int64_t)k * per);
-    const int c = cr / L.rows, r = cr - c * L.rows;
     const kk_fp_angle* P = L.angles + L.rec0 + k;
+    const int A = __ldg(&P->axis);
+    const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
+    const bool shared = shared_record(P, A, D1);
     float src[3], cor[3], u[3], v[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -83,14 +112,27 @@ __global__ void fpt_rays_kernel(const FptArgs L) {
         u[q] = __ldg(&P->u[q]);
         v[q] = __ldg(&P->v[q]);
     }
-    const int A = __ldg(&P->axis);
-    const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
-    const RaySetup R = ray_setup(src, cor, u, v, A, D1, D2, r, c, L.os[3 * A], L.os[3 * A + 1]);
     const int a = __ldg(&P->index);
     const float* plane = L.table ? (const float*)L.table[a] : L.proj + (int64_t)a * L.ps[0];
-    const float p = __ldg(plane + (int64_t)r * L.ps[1] + (int64_t)c * L.ps[2]);
-    L.ray_ab[id] = make_float4(R.a1, R.b1, R.a2, R.b2);
-    L.ray_pc[id] = p * (R.corr * L.os[3 * A + 2]);
+    auto value = [&](const RaySetup& R, int r, int c) {
+        return __ldg(plane + (int64_t)r * L.ps[1] + (int64_t)c * L.ps[2]) * (R.corr * L.os[3 * A + 2]);
+    };
+    const RayRecord O = ray_record(L, k);
+    if (shared) {
+        const int pos = cr / L.cols, c = cr % L.cols;
+        const bool up = pick3(v, D2) >= 0.f;
+        const int r0 = up ? pos : L.rows - 1 - pos;
+        const int r1 = up ? min(pos + 1, L.rows - 1) : max(r0 - 1, 0);
+        const RaySetup R = ray_setup(src, cor, u, v, A, D1, D2, r0, c, L.os[3 * A], L.os[3 * A + 1]);
+        const RaySetup Q = ray_setup(src, cor, u, v, A, D1, D2, r1, c, L.os[3 * A], L.os[3 * A + 1]);
+        O.ab[cr] = make_float4(R.a2, Q.a2, value(R, r0, c), value(Q, r1, c));
+        if (pos == 0) O.pc[c] = R.a1;
+    } else {
+        const int r = cr % L.rows, c = cr / L.rows;
+        const RaySetup R = ray_setup(src, cor, u, v, A, D1, D2, r, c, L.os[3 * A], L.os[3 * A + 1]);
+        O.pc[cr] = value(R, r, c);
+        O.ab[cr] = make_float4(R.a1, R.b1, R.a2, R.b2);
+    }
 }
 
 // A ray's in-slice coordinate at slice off + nst: the slab-start value v0
@@ -187,20 +229,10 @@ __device__ __forceinline__ bool footprint_box(const FptArgs& L, const kk_fp_angl
     return false;
 }
 
-// circular scans: the detector's v has no component along A and D1, so
-// every row of a column has bit for bit the same D1 coordinate sequence
-// (as in the forward projector's shared path)
-__device__ __forceinline__ bool shared_record(const kk_fp_angle* P, int A, int D1) {
-    const float vA = A == 0 ? __ldg(&P->v[0]) : (A == 1 ? __ldg(&P->v[1]) : __ldg(&P->v[2]));
-    const float vD1 = D1 == 0 ? __ldg(&P->v[0]) : __ldg(&P->v[1]);
-    return vA == 0.f && vD1 == 0.f;
-}
-
 // Contribution of record k of the chunk to voxel (w0, w1, w2): every pixel
 // of the voxel's candidate box is tested exactly.
 template <bool TEX8>
 __device__ float gather_record(const FptArgs& L, int k, int w0, int w1, int w2) {
-    const int64_t per = (int64_t)L.rows * L.cols;
     const kk_fp_angle* P = L.angles + L.rec0 + k;
     const int A = __ldg(&P->axis);
     const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
@@ -222,47 +254,37 @@ __device__ float gather_record(const FptArgs& L, int k, int w0, int w1, int w2) 
                   (float)kv + 1.5f - half2, c0, c1, rlo, rhi);
     const int off = (s / L.slab) * L.slab;
     const float t1 = __fadd_rn(__fsub_rn((float)off, 0.5f * (float)nS), 0.5f);
-    const bool shared = shared_record(P, A, D1);
     const int nst = s - off;
+    const RayRecord O = ray_record(L, k);
     float acc = 0.f;
     for (int c = c0; c <= c1; ++c) {
-        // shared case: one D1 coordinate for the whole column
-        Split syc;
-        bool col = false;
-        if (shared && rlo <= rhi) {
-            const float4 ab = __ldg(&L.ray_ab[(int64_t)k * per + (int64_t)c * L.rows + rlo]);
-            syc = split_coord<TEX8>(slice_coord<TEX8>(__fadd_rn(fmaf(ab.x, t1, ab.y), half1), ab.x, nst));
-            if ((unsigned)(jv - syc.i) > 1u) continue;
-            col = true;
-        }
         for (int r = rlo; r <= rhi; ++r) {
-            const int64_t id = (int64_t)k * per + (int64_t)c * L.rows + r;
-            const float4 ab = __ldg(&L.ray_ab[id]);
+            const int64_t id = (int64_t)c * L.rows + r;
+            const float4 ab = __ldg(&O.ab[id]);
             // the forward projector's coordinates for slice s
-            const Split sy =
-                col ? syc : split_coord<TEX8>(slice_coord<TEX8>(__fadd_rn(fmaf(ab.x, t1, ab.y), half1), ab.x, nst));
+            const Split sy = split_coord<TEX8>(slice_coord<TEX8>(__fadd_rn(fmaf(ab.x, t1, ab.y), half1), ab.x, nst));
             const Split sz = split_coord<TEX8>(slice_coord<TEX8>(__fadd_rn(fmaf(ab.z, t1, ab.w), half2), ab.z, nst));
             const int di = jv - sy.i, dj = kv - sz.i;
             if ((unsigned)di > 1u || (unsigned)dj > 1u) continue;
             const W4 wt = weights4<TEX8>(sy.w, sz.w, rule, a_fast);
             float wgt = di == 0 ? (dj == 0 ? wt.w00 : wt.w01) : (dj == 0 ? wt.w10 : wt.w11);
             if (TEX8) wgt *= 1.f / 256.f;
-            acc = fmaf(__ldg(&L.ray_pc[id]), wgt, acc);
+            acc = fmaf(__ldg(&O.pc[id]), wgt, acc);
         }
     }
     return acc;
 }
 
-// General path: one thread per voxel, every record of the chunk (except
-// those a tile pass handles, when L.tiled says so).
+// General path: one thread per voxel, every record of the chunk that the
+// column passes do not handle.
 template <bool TEX8>
 __global__ void __launch_bounds__(FPT_TILE_2* FPT_TILE_1) fpt_gather_kernel(const FptArgs L) {
-    // nothing to do when the tile passes handle every record of the chunk
+    // nothing to do when the column passes handle every record of the chunk
     int todo = 0;
     for (int k = threadIdx.y * FPT_TILE_2 + threadIdx.x; k < L.nrec; k += FPT_TILE_2 * FPT_TILE_1) {
         const kk_fp_angle* P = L.angles + L.rec0 + k;
         const int A = __ldg(&P->axis);
-        if (!(L.tiled[A] && shared_record(P, A, A == 1 ? 0 : 1))) todo = 1;
+        if (!shared_record(P, A, A == 1 ? 0 : 1)) todo = 1;
     }
     if (!__syncthreads_or(todo)) return;
     const int i2 = blockIdx.x * FPT_TILE_2 + threadIdx.x;
@@ -277,7 +299,7 @@ __global__ void __launch_bounds__(FPT_TILE_2* FPT_TILE_1) fpt_gather_kernel(cons
     for (int k = 0; k < L.nrec; ++k) {
         const kk_fp_angle* P = L.angles + L.rec0 + k;
         const int A = __ldg(&P->axis);
-        if (L.tiled[A] && shared_record(P, A, A == 1 ? 0 : 1)) continue;
+        if (shared_record(P, A, A == 1 ? 0 : 1)) continue;
         acc += gather_record<TEX8>(L, k, w0, w1, w2);
     }
     float* out = L.vol + (int64_t)w0 * L.vs[0] + (int64_t)w1 * L.vs[1] + (int64_t)w2 * L.vs[2];
@@ -285,52 +307,77 @@ __global__ void __launch_bounds__(FPT_TILE_2* FPT_TILE_1) fpt_gather_kernel(cons
 }
 
 // ---------------------------------------------------------------------------
-// tile pass for circular scans
+// column pass for circular scans
 // ---------------------------------------------------------------------------
-// One block owns a FPT_TJ x FPT_TK tile of texels (along D1, D2) of one
-// slice of the records whose dominant axis is A and whose rows share their
-// D1 coordinate. Per record it (1) finds the candidate columns and rows of
-// the tile's footprint, (2) computes every candidate column's D1 split and
-// every candidate ray's D2 split with the forward projector's own
-// slab-restart sequence, and stores the ray's four contributions
-// p * corr * outputScale * weight (one per texel of its bilinear
-// footprint) in shared memory, with per-(column, texel row) tables of the
-// rays that touch each row, then (3) every texel sums the contributions of
-// the rays that touch it. Each ray is set up once per tile instead of once
-// per voxel it might touch, and each texel reads only its own ~9 terms.
-// Records whose footprint exceeds the tables take the per-voxel path.
-constexpr int FPT_TJ = 16, FPT_TK = 32;    // texels of a tile along D1, D2
-constexpr int FPT_MAXC = 40, FPT_MAXR = 72;  // candidate columns, rows
-constexpr int FPT_THREADS = 256;
-constexpr size_t FPT_SMEM = (size_t)FPT_MAXC * FPT_MAXR * (sizeof(float4) + sizeof(int)) +
-                            (size_t)FPT_MAXC * (FPT_TK + 1) * 2 * sizeof(int) + (size_t)FPT_MAXC * 2 * sizeof(int) +
-                            (size_t)(FPT_TJ + 1) * 2 * sizeof(int);
+// Records whose dominant axis is A and whose rows share their D1
+// coordinate. One warp owns FPC_TJ rows (along D1) x FPC_TK texels (along
+// D2) of one slice and keeps their sums in registers, a lane per row, while
+// it walks the records. Work is laid out so that every ray is set up once
+// per warp and nothing is tested per texel:
+//
+//   * the detector columns whose D1 texel pair {i1, i1 + 1} meets the rows
+//     are packed over the lanes, 32 (record, column) pairs at a time across
+//     record boundaries, so the lanes stay busy whatever a record's share;
+//   * down its column a lane's D2 coordinate only grows, so the texels are
+//     visited in order (unrolled: the sums' register is static) and each
+//     takes the lane's next rays, evaluated two at a time in paired FP32,
+//     as long as their left texel is the current one. A ray adds to the
+//     current texel and to the carry of the next, for both texel rows: its
+//     four weights, exactly the forward projector's;
+//   * the two sums of the columns (rows i1 and i1 + 1) then move to the
+//     rows' lanes by shuffles whose sources are found once per 32 pairs.
+//
+// Lane 0 is the row before the first owned one: it only hands its second
+// row's sums on. A column whose D2 step per detector row is below 1/16
+// texel or above 1024 texels, or not finite, is handed round the warp and
+// tested ray by ray.
+//
+// Bound by instruction issue (about 115 warp instructions per 32 (column,
+// texel) pairs, 76 % of the issue slots used) and then by the latency of
+// the ray loads. 256^3 x 360 x 384^2: 256.5 -> 36.8 ms against a per-texel
+// gather from shared-memory tables, 64^3 x 96 x 96^2: 1.60 -> 0.37 ms. The
+// sums live in shared memory, not in registers: a register per texel means
+// unrolling the texel loop, whose code then misses the instruction cache
+// (75 ms).
+constexpr int FPC_TJ = 31;
+constexpr int FPC_TK = 32;
+constexpr int FPC_LD = 33;  // stride of a warp's sums: rows are read back along D2
 
-template <bool TEX8>
-__global__ void __launch_bounds__(FPT_THREADS) fpt_tile_kernel(const FptArgs L, int A) {
-    extern __shared__ __align__(16) unsigned char fpt_sm[];
-    float4* contrib = reinterpret_cast<float4*>(fpt_sm);
-    int* ri2 = reinterpret_cast<int*>(contrib + FPT_MAXC * FPT_MAXR);
-    int* rlo = ri2 + FPT_MAXC * FPT_MAXR;
-    int* rhi = rlo + FPT_MAXC * (FPT_TK + 1);
-    int* ci1 = rhi + FPT_MAXC * (FPT_TK + 1);
-    float* cS = reinterpret_cast<float*>(ci1 + FPT_MAXC);
-    int* clo = reinterpret_cast<int*>(cS + FPT_MAXC);
-    int* chi = clo + (FPT_TJ + 1);
-    // candidate box per record of the current group: first column, columns,
-    // first row, rows (columns <= 0: the record does not touch the tile, or
-    // is not this pass'; columns > FPT_MAXC or rows > FPT_MAXR: per voxel)
-    __shared__ int4 s_box[FPT_THREADS];
+// weight rule of a pass: any (weights4), or the two rules of a D2 axis
+// faster than D1
+enum FpcRule { FPC_ANY = 0, FPC_RULE0 = 1, FPC_RULE1 = 2 };
 
+// n rounded adds of a slope, n the same for the whole warp.
+template <typename T, typename Add>
+__device__ __forceinline__ T add_steps(T v, T a, int n, Add add) {
+    for (int q = n >> 4; q > 0; --q) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v = add(v, a);
+    }
+    if (n & 8) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v = add(v, a);
+    }
+    if (n & 4) v = add(add(add(add(v, a), a), a), a);
+    if (n & 2) v = add(add(v, a), a);
+    if (n & 1) v = add(v, a);
+    return v;
+}
+
+template <bool TEX8, int RULE, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 36 / WARPS) fpt_column_kernel(const FptArgs L, int A) {
+    __shared__ unsigned s_rows[WARPS][32];
+    __shared__ float s_acc[WARPS][FPC_TK * FPC_LD];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
     const int nS = L.vn[A], n1 = L.vn[D1], n2 = L.vn[D2];
-    // slices fastest: the blocks in flight cover few tiles at many slices,
-    // which read nearly the same rays, so the ray set-ups are re-read from
-    // L2 instead of DRAM
-    const int ktiles = (n2 + FPT_TK - 1) / FPT_TK;
+    // the block's warps share the records (which alternate between the axes
+    // in small groups: a warp's place among WARPS rotates). Slices fastest:
+    // the blocks in flight read nearly the same rays
+    const int ktiles = (n2 + FPC_TK - 1) / FPC_TK;
     const int s = blockIdx.x % nS, tile = blockIdx.x / nS;
-    const int j0 = (tile / ktiles) * FPT_TJ, k0 = (tile % ktiles) * FPT_TK;
-    const int tid = threadIdx.x;
+    const int j0 = (tile / ktiles) * FPC_TJ, k0 = (tile % ktiles) * FPC_TK;
     const float half1 = 0.5f * (float)n1, half2 = 0.5f * (float)n2;
     const int rule = 2 - L.rank[A];
     const bool a_fast = L.rank[D1] < L.rank[D2];
@@ -338,137 +385,240 @@ __global__ void __launch_bounds__(FPT_THREADS) fpt_tile_kernel(const FptArgs L, 
     const float t1 = __fadd_rn(__fsub_rn((float)off, 0.5f * (float)nS), 0.5f);
     const int nst = s - off;
     const float t = (float)s - 0.5f * (float)nS + 0.5f;
-    const int64_t per = (int64_t)L.rows * L.cols;
-    // this thread's texels: (j0 + tt / FPT_TK, k0 + tt % FPT_TK), tt = tid, tid + 256
-    int tj[2], tk[2];
-    float acc[2] = {0.f, 0.f};
+    const int rows = L.rows, cols = L.cols;
+    auto add1 = [](float a, float b) { return __fadd_rn(a, b); };
+    auto addp = [](float2 a, float2 b) { return add2(a, b); };
+
+    float* acc = &s_acc[warp][lane];  // texel kk of this lane's row: acc[FPC_LD kk]
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int tt = tid + q * FPT_THREADS;
-        tj[q] = j0 + tt / FPT_TK;
-        tk[q] = k0 + tt % FPT_TK;
-    }
-    auto world = [&](int q, int& w0, int& w1, int& w2) {
-        const int j = min(tj[q], n1 - 1), kk = min(tk[q], n2 - 1);
-        w0 = A == 0 ? s : (D1 == 0 ? j : kk);
-        w1 = A == 1 ? s : (D1 == 1 ? j : kk);
-        w2 = A == 2 ? s : (D2 == 2 ? kk : j);
-    };
-    for (int g0 = 0; g0 < L.nrec; g0 += FPT_THREADS) {
-        // the candidate boxes of up to 256 records at once, one per thread
-        const int gn = min(FPT_THREADS, L.nrec - g0);
-        __syncthreads();  // the previous group's boxes are no longer read
-        if (tid < gn) {
-            const kk_fp_angle* P = L.angles + L.rec0 + g0 + tid;
-            int4 bx = make_int4(0, 0, 0, 0);
+    for (int q = 0; q < FPC_TK; ++q) acc[FPC_LD * q] = 0.f;
+    auto record = [&](int i) { return i * WARPS + ((warp + 3 * i) & (WARPS - 1)); };
+    bool touched = false;
+
+    for (int g0 = 0; g0 * WARPS < L.nrec; g0 += 32) {
+        // the candidate columns of 32 records, one per lane
+        int first = 0, cnt = 0;
+        if (record(g0 + lane) < L.nrec) {
+            const kk_fp_angle* P = L.angles + L.rec0 + record(g0 + lane);
             if (__ldg(&P->axis) == A && shared_record(P, A, D1)) {
                 int c0, c1, rl, rh;
-                footprint_box(L, P, A, D1, t, (float)j0 - 0.5f - half1, (float)(j0 + FPT_TJ) + 0.5f - half1,
-                              (float)k0 - 0.5f - half2, (float)(k0 + FPT_TK) + 0.5f - half2, c0, c1, rl, rh);
-                bx = make_int4(c0, c1 >= c0 && rh >= rl ? c1 - c0 + 1 : 0, rl, rh - rl + 1);
+                footprint_box(L, P, A, D1, t, (float)j0 - 0.5f - half1, (float)(j0 + FPC_TJ) + 0.5f - half1,
+                              (float)k0 - 0.5f - half2, (float)(k0 + FPC_TK) + 0.5f - half2, c0, c1, rl, rh);
+                first = c0;
+                cnt = rh >= rl ? max(c1 - c0 + 1, 0) : 0;
             }
-            s_box[tid] = bx;
         }
-        __syncthreads();
-        for (int kq = 0; kq < gn; ++kq) {
-            const int k = g0 + kq;
-            const int4 bx = s_box[kq];
-            const int c0 = bx.x, nc = bx.y, r0 = bx.z, nr = bx.w;
-            if (nc <= 0) continue;  // uniform
-            if (nc > FPT_MAXC || nr > FPT_MAXR) {  // beyond the tables: per voxel
+        int incl = cnt;
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    int w0, w1, w2;
-                    world(q, w0, w1, w2);
-                    acc[q] += gather_record<TEX8>(L, k, w0, w1, w2);
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(full, incl, d);
+            if (lane >= d) incl += v;
+        }
+        const int total = __shfl_sync(full, incl, 31);
+        first -= incl - cnt;  // column of flat index f: first + f
+        touched = touched || total > 0;
+        for (int b = 0; b < total; b += 32) {
+            // this lane's (record, column)
+            const int f = b + lane;
+            int m = 0;
+#pragma unroll
+            for (int d = 16; d >= 1; d >>= 1)
+                if (__shfl_sync(full, incl, m + d - 1) <= f) m += d;
+            const int c = __shfl_sync(full, first, m) + f;
+            const RayRecord O = ray_record(L, record(g0 + m));
+            const float4* ray = O.ab + c;  // position 0 of the column
+            // its D1 split, and its D2 coordinate at the first and last ray
+            Split sy;
+            sy.i = 0;
+            sy.w = 0.f;
+            bool in = f < total, ok = true;
+            float z0 = 0.f, dz = 1.f, sA = 0.f, s2 = 0.f;
+            if (in) {
+                const kk_fp_angle* P = L.angles + L.rec0 + record(g0 + m);
+                const float a1 = __ldg(&O.pc[c]);
+                sA = __ldg(&P->src[A]);
+                s2 = __ldg(&P->src[D2]);
+                const float b1 = fmaf(-a1, sA, __ldg(&P->src[D1]));  // as ray_setup
+                const float y = add_steps(__fadd_rn(fmaf(a1, t1, b1), half1), a1, nst, add1);
+                sy = split_coord<TEX8>(y);
+                in = (unsigned)(sy.i - (j0 - 1)) < 32u;
+                const float e0 = __ldg(&ray->x), e1 = __ldg(&ray[(int64_t)(rows - 1) * cols].x);
+                z0 = fmaf(e0, t, fmaf(-e0, sA, s2)) + half2;
+                const float z1 = fmaf(e1, t, fmaf(-e1, sA, s2)) + half2;
+                dz = rows > 1 ? (z1 - z0) / (float)(rows - 1) : 1.f;
+                ok = fabsf(dz) >= 0.0625f && fabsf(dz) <= 1024.f && isfinite(z0);
+                if (dz < 0.f) z0 = z1;
+            }
+            const int v1 = sy.i - (j0 - 1);
+            // the lanes of each row
+            s_rows[warp][lane] = 0;
+            __syncwarp();
+            const unsigned peers = __match_any_sync(full, in && ok ? v1 : -1);
+            if (in && ok && lane == __ffs(peers) - 1) s_rows[warp][v1] = peers;
+            __syncwarp();
+            const unsigned mine = s_rows[warp][lane], rest = mine & (mine - 1);
+            __syncwarp();
+            const int most = __reduce_max_sync(full, __popc(mine));
+            const int l0 = __ffs(mine) - 1, l1 = __ffs(rest) - 1;
+            // Walks the columns' rays in order of growing D2. BACK: some lane
+            // meets them from the last position (a slice behind the source).
+            auto walk = [&](auto back_tag) {
+                constexpr bool BACK = decltype(back_tag)::value;
+                // start two or less before the first ray whose left texel
+                // may be k0 - 1
+                const bool back = BACK && dz < 0.f;
+                const float pf = floorf(((float)k0 - 0.5f - z0) / fabsf(dz)) - 1.f;
+                int left = in && ok ? rows - (int)fminf(fmaxf(pf, 0.f), (float)rows) : 0;  // rays from here on
+                // lanes without rays keep reading an entry that exists
+                const float S = sy.w, S256 = S * (1.f / 256.f);
+                const float4* rp = left > 0 ? ray + (int64_t)(rows - left) * cols : L.ray_ab;
+                int ia, ib;  // left texels of the next two rays, from k0
+                float2 F, pc;
+                auto eval = [&]() {
+                    float4 e = __ldg(!BACK || left <= 0 || !back ? rp : ray + (int64_t)max(left - 2, 0) * cols);
+                    if (BACK && back && left > 1) e = make_float4(e.y, e.x, e.w, e.z);
+                    pc = f2(e.z, e.w);
+                    const float2 a2 = f2(e.x, e.y);
+                    // slab start as the forward projector: (a2 t1 + b2) + half2
+                    const float2 z = add_steps(add2(fma2(a2, f2(t1), fma2(a2, f2(-sA), f2(s2))), f2(half2)), a2, nst, addp);
+                    if (TEX8) {
+                        const float2 q = add2_rd(fma2_rd(z, f2(256.f), f2(-127.5f)), f2(12582912.f));
+                        const int b0 = __float_as_int(q.x), b1 = __float_as_int(q.y);
+                        ia = b0 >> 8;
+                        ib = b1 >> 8;
+                        F = add2(f2(__int_as_float((b0 & 255) | 0x4B000000), __int_as_float((b1 & 255) | 0x4B000000)),
+                                 f2(-8388608.f));
+                    } else {
+                        const Split sa = split_coord<false>(z.x), sb = split_coord<false>(z.y);
+                        ia = sa.i;
+                        ib = sb.i;
+                        F = f2(left > 0 ? sa.w : 0.f, left > 1 ? sb.w : 0.f);
+                    }
+                };
+                auto advance = [&](int n) {
+                    left -= n;
+                    if (left > 0) rp += n * cols;
+                };
+                auto weights = [&](float2& w00, float2& w01, float2& w10, float2& w11) {
+                    if (RULE == FPC_ANY || !TEX8) {
+                        const W4 a = weights4<TEX8>(S, F.x, rule, a_fast), b = weights4<TEX8>(S, F.y, rule, a_fast);
+                        w00 = f2(a.w00, b.w00);
+                        w01 = f2(a.w01, b.w01);
+                        w10 = f2(a.w10, b.w10);
+                        w11 = f2(a.w11, b.w11);
+                    } else {
+                        // x1 = round half up(F S / 256), x0 as weights4
+                        w11 = add2(add2_rd(fma2(F, f2(S256), f2(0.5f)), f2(12582912.f)), f2(-12582912.f));
+                        w01 = RULE == FPC_RULE1 ? add2(add2_rd(fma2(F, f2(-S256), f2(0.5f)), f2(12582912.f)),
+                                                       add2(F, f2(-12582912.f)))
+                                                : sub2(F, w11);
+                        w00 = sub2(f2(256.f - S), w01);
+                        w10 = sub2(f2(S), w11);
+                    }
+                };
+                const int base = k0 + (TEX8 ? 0x4B4000 : 0);  // texel k0 as eval numbers it
+                eval();
+                while (__any_sync(full, left > 0 && ia < base - 1)) {
+                    advance((left > 0 && ia < base - 1) + (left > 1 && ib < base - 1));
+                    eval();
                 }
-                continue;
-            }
-            for (int i = tid; i < nc * (FPT_TK + 1); i += FPT_THREADS) {
-                rlo[i] = 1;
-                rhi[i] = 0;
-            }
-            if (tid < FPT_TJ + 1) {
-                clo[tid] = 1;
-                chi[tid] = 0;
-            }
-            // (1) the D1 split of every candidate column
-            for (int c = tid; c < nc; c += FPT_THREADS) {
-                const float4 ab = __ldg(&L.ray_ab[(int64_t)k * per + (int64_t)(c0 + c) * L.rows + r0]);
-                const Split sy =
-                    split_coord<TEX8>(slice_coord<TEX8>(__fadd_rn(fmaf(ab.x, t1, ab.y), half1), ab.x, nst));
-                ci1[c] = sy.i;
-                cS[c] = sy.w;
-            }
-            __syncthreads();
-            // the columns of each texel row: the D1 split is monotone in
-            // the column, so each row's columns are a range, whose ends are
-            // where the split changes (tables are empty where none)
-            for (int c = tid; c < nc; c += FPT_THREADS) {
-                const int v = ci1[c] - (j0 - 1);
-                if (v < 0 || v > FPT_TJ) continue;
-                if (c == 0 || ci1[c - 1] != ci1[c]) clo[v] = c;
-                if (c == nc - 1 || ci1[c + 1] != ci1[c]) chi[v] = c;
-            }
-            // (2) every candidate ray: its D2 split and its four contributions
-            for (int i = tid; i < nc * nr; i += FPT_THREADS) {
-                const int c = i / nr;
-                const int64_t id = (int64_t)k * per + (int64_t)(c0 + c) * L.rows + (r0 + i - c * nr);
-                const float4 ab = __ldg(&L.ray_ab[id]);
-                const Split sz =
-                    split_coord<TEX8>(slice_coord<TEX8>(__fadd_rn(fmaf(ab.z, t1, ab.w), half2), ab.z, nst));
-                const W4 wt = weights4<TEX8>(cS[c], sz.w, rule, a_fast);
-                const float pc = __ldg(&L.ray_pc[id]) * (TEX8 ? 1.f / 256.f : 1.f);
-                contrib[i] = make_float4(pc * wt.w00, pc * wt.w01, pc * wt.w10, pc * wt.w11);
-                ri2[i] = sz.i;
-            }
-            __syncthreads();
-            // the rows of each (column, texel row): ranges again, ends where
-            // the D2 split changes along the column
-            for (int i = tid; i < nc * nr; i += FPT_THREADS) {
-                const int c = i / nr, r = i - c * nr;
-                const int v = ri2[i] - (k0 - 1);
-                if (v < 0 || v > FPT_TK) continue;
-                if (r == 0 || ri2[i - 1] != ri2[i]) rlo[c * (FPT_TK + 1) + v] = r;
-                if (r == nr - 1 || ri2[i + 1] != ri2[i]) rhi[c * (FPT_TK + 1) + v] = r;
-            }
-            __syncthreads();
-            // (3) every texel sums the rays that touch it (each candidate is
-            // checked, so a split that is not monotone only costs time)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int j = tj[q], kk = tk[q];
-                float sum = 0.f;
-#pragma unroll
-                for (int di = 0; di < 2; ++di) {
-                    const int vj = j - di;  // the ray's D1 texel: j (di = 0) or j - 1 (di = 1)
-                    const int cv = vj - (j0 - 1);
-                    for (int c = clo[cv]; c <= chi[cv]; ++c) {
-                        if (ci1[c] != vj) continue;
-#pragma unroll
-                        for (int dj = 0; dj < 2; ++dj) {
-                            const int vk = kk - dj;
-                            const int rv = c * (FPT_TK + 1) + vk - (k0 - 1);
-                            for (int r = rlo[rv]; r <= rhi[rv]; ++r) {
-                                const int i = c * nr + r;
-                                if (ri2[i] != vk) continue;
-                                sum += reinterpret_cast<const float*>(&contrib[i])[di * 2 + dj];
+                float2 n0 = f2(0.f), n1s = f2(0.f);  // carries of the next texel, rows i1 and i1 + 1
+                float* ak = acc - FPC_LD;
+#pragma unroll 1
+                for (int kk = base - 1; kk < base + FPC_TK; ++kk, ak += FPC_LD) {
+                    bool ta = left > 0 && ia == kk, tb = left > 1 && ib == kk;
+                    float2 w = f2(ta ? pc.x : 0.f, tb ? pc.y : 0.f), w00, w01, w10, w11;
+                    weights(w00, w01, w10, w11);
+                    float2 g0s = fma2(w, w00, n0), g1s = fma2(w, w10, n1s);
+                    n0 = mul2(w, w01);
+                    n1s = mul2(w, w11);
+                    advance((int)ta + (int)tb);
+                    eval();
+                    // more than two rays of this texel
+                    while (__any_sync(full, ta = left > 0 && ia == kk)) {
+                        tb = left > 1 && ib == kk;
+                        w = f2(ta ? pc.x : 0.f, tb ? pc.y : 0.f);
+                        weights(w00, w01, w10, w11);
+                        g0s = fma2(w, w00, g0s);
+                        n0 = fma2(w, w01, n0);
+                        g1s = fma2(w, w10, g1s);
+                        n1s = fma2(w, w11, n1s);
+                        advance((int)ta + (int)tb);
+                        eval();
+                    }
+                    if (kk < base) continue;
+                    const float G0 = g0s.x + g0s.y, G1 = g1s.x + g1s.y;
+                    float h0 = 0.f, h1 = 0.f;
+                    const float a0 = __shfl_sync(full, G0, l0), a1 = __shfl_sync(full, G1, l0);
+                    const float c0 = __shfl_sync(full, G0, l1), c1 = __shfl_sync(full, G1, l1);
+                    if (mine) {
+                        h0 = a0;
+                        h1 = a1;
+                    }
+                    if (rest) {
+                        h0 += c0;
+                        h1 += c1;
+                    }
+                    if (most > 2) {
+                        unsigned more = rest & (rest - 1);
+                        for (int q = 2; q < most; ++q) {
+                            const int l = __ffs(more) - 1;
+                            const float d0 = __shfl_sync(full, G0, l), d1 = __shfl_sync(full, G1, l);
+                            if (more) {
+                                h0 += d0;
+                                h1 += d1;
                             }
+                            more &= more - 1;
                         }
                     }
+                    *ak += h0 + __shfl_up_sync(full, h1, 1);
                 }
-                acc[q] += sum;
+            };
+            if (most > 0) {
+                if (__any_sync(full, in && ok && dz < 0.f))
+                    walk(std::true_type{});
+                else
+                    walk(std::false_type{});
             }
-            __syncthreads();  // the tables are rebuilt for the next record
+            // columns that cannot be walked: every ray against every texel
+            unsigned odd = __ballot_sync(full, in && !ok);
+            while (odd) {
+                const int l = __ffs(odd) - 1;
+                odd &= odd - 1;
+                const int cq = __shfl_sync(full, c, l), vq = __shfl_sync(full, v1, l);
+                const float4* rq = ray_record(L, record(g0 + __shfl_sync(full, m, l))).ab + cq;
+                const float S = __shfl_sync(full, sy.w, l);
+                const float qA = __shfl_sync(full, sA, l), q2 = __shfl_sync(full, s2, l);
+                const int dj = lane - vq;  // this lane's row: i1 (0) or i1 + 1 (1)
+                for (int r = 0; (unsigned)dj < 2u && r < rows; ++r) {
+                    const float4 ab = __ldg(rq + (int64_t)r * cols);
+                    const float z =
+                        add_steps(__fadd_rn(fmaf(ab.x, t1, fmaf(-ab.x, qA, q2)), half2), ab.x, nst, add1);
+                    const Split sz = split_coord<TEX8>(z);
+                    const int kk = sz.i - k0;
+                    const W4 w = weights4<TEX8>(S, sz.w, rule, a_fast);
+                    if (kk >= 0 && kk < FPC_TK) acc[FPC_LD * kk] += ab.z * (dj ? w.w10 : w.w00);
+                    if (kk >= -1 && kk < FPC_TK - 1) acc[FPC_LD * (kk + 1)] += ab.z * (dj ? w.w11 : w.w01);
+                }
+            }
+            __syncwarp();
         }
     }
+    touched = __syncthreads_or(touched);
+    if (!touched && L.accumulate) return;
+    // lanes along the faster of the two axes
+    const bool along2 = L.rank[D2] < L.rank[D1];
+    float* out = L.vol + (int64_t)s * L.vs[A];
+    for (int q = warp; q < 32; q += WARPS) {
+        const int row = along2 ? q : lane, kk = along2 ? lane : q;
+        const int j = j0 - 1 + row, k = k0 + kk;
+        if (row == 0 || j >= n1 || k >= n2) continue;
+        float v = s_acc[0][kk * FPC_LD + row];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        if (tj[q] >= n1 || tk[q] >= n2) continue;
-        int w0, w1, w2;
-        world(q, w0, w1, w2);
-        float* out = L.vol + (int64_t)w0 * L.vs[0] + (int64_t)w1 * L.vs[1] + (int64_t)w2 * L.vs[2];
-        *out = L.accumulate ? *out + acc[q] : acc[q];
+        for (int w = 1; w < WARPS; ++w) v += s_acc[w][kk * FPC_LD + row];
+        v *= 1.f / weight_unit<TEX8>();
+        float* o = out + (int64_t)j * L.vs[D1] + (int64_t)k * L.vs[D2];
+        *o = L.accumulate ? *o + v : v;
     }
 }
 
@@ -478,6 +628,42 @@ __global__ void __launch_bounds__(FPT_THREADS) fpt_tile_kernel(const FptArgs L, 
 // host side
 // ===========================================================================
 using namespace kk;
+
+template <int WARPS>
+static void launch_column_split(const FptArgs& L, int A, bool tex8, cudaStream_t st) {
+    const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
+    constexpr int threads = 32 * WARPS;
+    // below 2^31 for every volume the library takes (axes below 2^14)
+    const unsigned blocks = (unsigned)((int64_t)L.vn[A] * ((L.vn[D1] + FPC_TJ - 1) / FPC_TJ) *
+                                       ((L.vn[D2] + FPC_TK - 1) / FPC_TK));
+    // rules 0 and 1 with D2 the faster in-slice axis have their own code;
+    // the middle + slowest plane (rule 2) and permuted volumes go by weights4
+    const bool d2_fast = L.rank[D2] < L.rank[D1];
+    if (!tex8)
+        fpt_column_kernel<false, FPC_ANY, WARPS><<<blocks, threads, 0, st>>>(L, A);
+    else if (d2_fast && L.rank[A] == 2)
+        fpt_column_kernel<true, FPC_RULE0, WARPS><<<blocks, threads, 0, st>>>(L, A);
+    else if (d2_fast && L.rank[A] == 1)
+        fpt_column_kernel<true, FPC_RULE1, WARPS><<<blocks, threads, 0, st>>>(L, A);
+    else
+        fpt_column_kernel<true, FPC_ANY, WARPS><<<blocks, threads, 0, st>>>(L, A);
+}
+
+// The records are split over the warps of a block, which add their sums in
+// order: four ways (four slices' tiles take turns more evenly than one long
+// warp each: 256^3 x 360 x 384^2 41.1 -> 36.7 ms), eight ways while the
+// (slice, tile) pairs fill less than about four rounds of the GPU (128 x 128
+// x 100 x 180 2.60 -> 2.43 ms, 64^3 x 96 0.54 -> 0.37 ms; 192 x 192 x 180 x
+// 250, at 54 pairs per SM, 10.62 ms four ways and 10.88 eight ways).
+static void launch_column_pass(const FptArgs& L, int A, bool tex8, cudaStream_t st) {
+    const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
+    const int64_t pairs =
+        (int64_t)L.vn[A] * ((L.vn[D1] + FPC_TJ - 1) / FPC_TJ) * ((L.vn[D2] + FPC_TK - 1) / FPC_TK);
+    if (pairs < (int64_t)kk_sm_count() * 40)
+        launch_column_split<8>(L, A, tex8, st);
+    else
+        launch_column_split<4>(L, A, tex8, st);
+}
 
 extern "C" int kk_cone_fp_adjoint(const kk_projections* proj, const kk_volume* vol, const kk_fp_angle* angles,
                                   const float* out_scale, int32_t interp, int32_t slab, int32_t additive,
@@ -535,38 +721,20 @@ extern "C" int kk_cone_fp_adjoint(const kk_projections* proj, const kk_volume* v
     const dim3 block(FPT_TILE_2, FPT_TILE_1);
     const dim3 grid((L.vn[L.m2] + FPT_TILE_2 - 1) / FPT_TILE_2, (L.vn[L.m1] + FPT_TILE_1 - 1) / FPT_TILE_1, L.vn[L.m0]);
     const bool tex8 = interp == KK_INTERP_TEX8;
-    // the tile passes: one per ray axis A, over that axis' slices
-    for (int A = 0; A < 3; ++A) {
-        const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
-        L.tiled[A] = ((L.vn[D2] + FPT_TK - 1) / FPT_TK) * (int64_t)((L.vn[D1] + FPT_TJ - 1) / FPT_TJ) * L.vn[A] <
-                     0x7fffffffLL;
-    }
-    const void* tk = tex8 ? (const void*)fpt_tile_kernel<true> : (const void*)fpt_tile_kernel<false>;
-    rc = kk_allow_smem(tk, FPT_SMEM, who);
-    if (rc) return rc;
     for (int r0 = 0; r0 < n; r0 += ck) {
         L.rec0 = r0;
         L.nrec = std::min(ck, n - r0);
         const int first = (r0 > 0 || additive) ? 1 : 0;
         const int64_t rays = (int64_t)L.nrec * per;
         fpt_rays_kernel<<<(unsigned)((rays + 255) / 256), 256, 0, st>>>(L);
-        // every voxel is written by the first tile pass (even where no ray
-        // of its axis touches it), the later passes and the per-voxel
+        // every voxel is written by the first column pass (even where no
+        // ray of its axis touches it), the later passes and the per-voxel
         // gather of the remaining records add
-        bool written = false;
         for (int A = 0; A < 3; ++A) {
-            if (!L.tiled[A]) continue;
-            const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
-            const unsigned tg = (unsigned)(((L.vn[D2] + FPT_TK - 1) / FPT_TK) *
-                                           (int64_t)((L.vn[D1] + FPT_TJ - 1) / FPT_TJ) * L.vn[A]);
-            L.accumulate = written ? 1 : first;
-            if (tex8)
-                fpt_tile_kernel<true><<<tg, FPT_THREADS, FPT_SMEM, st>>>(L, A);
-            else
-                fpt_tile_kernel<false><<<tg, FPT_THREADS, FPT_SMEM, st>>>(L, A);
-            written = true;
+            L.accumulate = A > 0 ? 1 : first;
+            launch_column_pass(L, A, tex8, st);
         }
-        L.accumulate = written ? 1 : first;
+        L.accumulate = 1;
         if (tex8)
             fpt_gather_kernel<true><<<grid, block, 0, st>>>(L);
         else
