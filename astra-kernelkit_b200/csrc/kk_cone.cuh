@@ -96,7 +96,9 @@ struct BpArgs {
 enum BpLoad { LOAD_ZERO = 0, LOAD_VOL = 1, LOAD_WORK = 2 };
 enum BpStore { STORE_VOL = 0, STORE_WORK = 1, STORE_FINAL = 2 };
 
-enum BpFetch { FETCH_GLOBAL = 0, FETCH_TEX = 1 };
+// texels from device memory, through the texture's own filter, or the four
+// texels of the footprint from the texture with exact weights
+enum BpFetch { FETCH_GLOBAL = 0, FETCH_TEX = 1, FETCH_GATHER = 2 };
 
 }  // namespace kk
 

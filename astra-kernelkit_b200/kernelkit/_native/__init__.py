@@ -56,6 +56,8 @@ class kk_fp_options(ctypes.Structure):
 #: kk_fp_options.flags: shared-memory tiles staged by the tensor-copy
 #: unit instead of direct loads for CUDA-core rays
 KK_FP_OPT_TILES = 1
+#: some records' detector rows do not share their in-slice coordinate
+KK_FP_OPT_GENERAL = 2
 
 
 class kk_bp_update(ctypes.Structure):
@@ -112,7 +114,8 @@ EXPORTS = ("kk_cone_fp_ex", "kk_fp_launches_ex", "kk_wait_timeouts",
            "kk_cone_bp_layered_batched",
            "kk_cone_bp", "kk_cone_bp_static",
            "kk_cone_bp_update", "kk_layered_create", "kk_layered_copy",
-           "kk_layered_destroy", "kk_cone_bp_layered",
+           "kk_layered_destroy", "kk_layered_fill", "kk_cone_bp_layered",
+           "kk_cone_bp_layered_ex",
            "kk_cone_bp_layered_update", "kk_preweight", "kk_filter_rows",
            "kk_reciprocal", "kk_sirt_update", "kk_fp_set_span",
            "kk_fp_launches", "kk_last_error",
@@ -166,6 +169,9 @@ def load():
     L.kk_layered_create.argtypes = [i64, i64, i64, i32, P(vp)]
     L.kk_layered_copy.argtypes = [vp, P(kk_projections), vp]
     L.kk_layered_destroy.argtypes = [vp]
+    L.kk_layered_fill.argtypes = [vp, P(kk_projections), i64, i64, vp]
+    L.kk_cone_bp_layered_ex.argtypes = [vp, i64, P(kk_volume), vp, f32, i32,
+                                        i32, vp, vp]
     L.kk_cone_bp_layered.argtypes = [vp, P(kk_volume), vp, f32, i32, vp, vp]
     L.kk_cone_bp_layered_update.argtypes = [vp, P(kk_volume), vp, f32,
                                             P(kk_bp_update), vp, vp]

@@ -190,16 +190,18 @@ typedef struct {
     void* padded;         /* NULL, or a device buffer of padded_elems
                              elements of the volume's type, at least
                              (n0 + 4)(n1 + 4)(n2 + 4) (no counterpart in the
-                             reference). With texture-compatible weights
-                             (and without KK_FP_OPT_TILES) the volume is
-                             copied into it at the start of the call with
+                             reference). Without KK_FP_OPT_TILES the volume
+                             is copied into it at the start of the call with
                              two zero texels before and after every axis,
                              and the rays are traced from that copy: the
-                             CUDA-core rays of circular scans then sample
+                             CUDA-core rays of circular scans (with
+                             KK_FP_OPT_GENERAL: of any scan) then sample
                              slabs that cross the volume's boundary with
                              the paired, test-free loads of the interior
                              (the zeros are the border), not the per-ray
-                             checked loop. Same results bit for bit. */
+                             checked loop. Same results bit for bit with
+                             texture-compatible weights; exact weights may
+                             round differently. */
     int64_t padded_elems; /* elements of padded */
 } kk_fp_options;
 
@@ -209,6 +211,12 @@ typedef struct {
  * measured shapes the per-slice pipeline costs more instructions than the
  * loads it replaces. */
 #define KK_FP_OPT_TILES 1
+/* kk_fp_options.flags, with padded: some records' detector rows do not
+ * share their in-slice coordinate (v has a component along the rays or the
+ * first in-slice axis: tilted detectors), so choose the kernel that pairs
+ * those rays too (same results; the other kernel keeps more rays in flight
+ * where every record shares). */
+#define KK_FP_OPT_GENERAL 2
 
 /* The forward projection with every option per call: kk_cone_fp,
  * kk_cone_fp_residual and kk_cone_fp_layered are this entry point with
@@ -323,6 +331,21 @@ KK_API int kk_layered_create(int64_t layers, int64_t height, int64_t width,
 KK_API int kk_layered_copy(kk_layered* tex, const kk_projections* src,
                            void* stream);
 KK_API int kk_layered_destroy(kk_layered* tex);
+
+/* Fill layers [0, count) from projections [first, first + count) of any
+ * layout (strides or a pointer table; float32), for callers that stage a
+ * scan through a texture of fewer layers. */
+KK_API int kk_layered_fill(kk_layered* tex, const kk_projections* src,
+                           int64_t first, int64_t count, void* stream);
+
+/* kk_cone_bp_layered on the first n_angles layers (0: all), with the
+ * texture's own interpolation (KK_INTERP_TEX8) or exact weights on its
+ * texels (KK_INTERP_EXACT; float32 texture and volume). */
+KK_API int kk_cone_bp_layered_ex(const kk_layered* tex, int64_t n_angles,
+                                 const kk_volume* vol,
+                                 const kk_bp_angle* angles, float out_scale,
+                                 int32_t interp, int32_t additive,
+                                 float* work, void* stream);
 
 /* kk_cone_bp / kk_cone_bp_update sampling the layered texture. */
 KK_API int kk_cone_bp_layered(const kk_layered* tex, const kk_volume* vol,
