@@ -40,6 +40,12 @@ namespace kk {
 #ifndef KK_FP_PAD_MINBLOCKS
 #define KK_FP_PAD_MINBLOCKS (40 / KK_FP_COLS)  // the padded-copy kernel: 48 registers, no spills
 #endif
+#ifndef KK_FP_GENERAL_MINBLOCKS
+#define KK_FP_GENERAL_MINBLOCKS (36 / KK_FP_COLS)
+#endif
+#ifndef KK_FP_EXACT_MINBLOCKS
+#define KK_FP_EXACT_MINBLOCKS (40 / KK_FP_COLS)
+#endif
 #ifndef KK_FP_PAD_TEX_UNROLL
 #define KK_FP_PAD_TEX_UNROLL 8  // its texture loop (4 in the 40-register kernel)
 #endif
@@ -126,7 +132,7 @@ __device__ __forceinline__ int span_class(float c0, float c1, int n) {
 }
 
 template <typename TV, typename TP, bool TEX8, int EPI, int PATH, int RULE, bool AF = false, bool SUMS = false,
-          bool PAD = false>
+          bool PAD = false, bool PAIR1 = false>
 __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, int rec, int a, int A, int D1, int D2,
                                          int rule, bool a_fast, int r0, int c, int lane) {
     float src[3], cor[3], u[3], v[3];
@@ -299,6 +305,106 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
                 shared_loop(std::false_type{});
             else if constexpr (PAD)
                 shared_loop(std::true_type{});
+        } else if (FP_RPT == 2 && PAD && (PATH == 2 || (PATH == 1 && PAIR1))) {
+            // The same for exact weights (floor by rounding down at 2^23)
+            // and for rays with D1 coordinates of their own (PATH 1), whose
+            // D1 splits are paired too.
+            auto pair_loop = [&](auto clamp_tag) {
+                constexpr bool CLAMP = decltype(clamp_tag)::value;
+                constexpr int BIAS = TEX8 ? 0x4B4000 : 0x4B400000;
+                float2 z2 = f2(zc[0], zc[1]), y2 = f2(yc[0], yc[1]), v2 = f2(0.f);
+                const float2 a2 = f2(R[0].a2, R[FP_RPT - 1].a2), a1 = f2(R[0].a1, R[FP_RPT - 1].a1);
+                const float yhi = (float)n1 + 1.49609375f, zhi = (float)n2 + 1.49609375f;
+                const TV* vol1 = vol + st1;
+                const int st1i = (int)st1, sSi = (int)sS;
+                int soff = off * sSi - BIAS;
+#pragma unroll FP_UNROLL
+                for (int sl = off; sl < end; ++sl, soff += sSi) {
+                    int r0, r1;  // row offsets of the two rays
+                    float2 S, S256;
+                    if (PATH == 2) {
+                        const float y = y2.x;
+                        const float ys = CLAMP ? fminf(fmaxf(y, -1.5f), yhi) : y;
+                        float s;
+                        if (TEX8) {
+                            const int yb = __float_as_int(__fadd_rd(__fmaf_rd(ys, 256.f, -127.5f), 12582912.f));
+                            r0 = ((yb >> 8) - 0x4B4000) * st1i + soff;
+                            s = __int_as_float((yb & 255) | 0x4B000000) - 8388608.f;
+                        } else {
+                            const float xb = ys - 0.5f, m = __fadd_rd(xb, 12582912.f);
+                            r0 = (__float_as_int(m) - BIAS) * st1i + soff;
+                            s = xb - (m - 12582912.f);
+                        }
+                        r1 = r0;
+                        S = f2(s);
+                        S256 = f2(s * (1.f / 256.f));
+                    } else {
+                        const float2 ys =
+                            CLAMP ? f2(fminf(fmaxf(y2.x, -1.5f), yhi), fminf(fmaxf(y2.y, -1.5f), yhi)) : y2;
+                        if (TEX8) {
+                            const float2 m = add2_rd(fma2_rd(ys, f2(256.f), f2(-127.5f)), f2(12582912.f));
+                            const int b0 = __float_as_int(m.x), b1 = __float_as_int(m.y);
+                            r0 = ((b0 >> 8) - 0x4B4000) * st1i + soff;
+                            r1 = ((b1 >> 8) - 0x4B4000) * st1i + soff;
+                            S = add2(f2(__int_as_float((b0 & 255) | 0x4B000000),
+                                        __int_as_float((b1 & 255) | 0x4B000000)), f2(-8388608.f));
+                            S256 = mul2(S, f2(1.f / 256.f));
+                        } else {
+                            const float2 xb = add2(ys, f2(-0.5f)), m = add2_rd(xb, f2(12582912.f));
+                            r0 = (__float_as_int(m.x) - BIAS) * st1i + soff;
+                            r1 = (__float_as_int(m.y) - BIAS) * st1i + soff;
+                            S = sub2(xb, add2(m, f2(-12582912.f)));
+                        }
+                    }
+                    const float2 zs =
+                        CLAMP ? f2(fminf(fmaxf(z2.x, -1.5f), zhi), fminf(fmaxf(z2.y, -1.5f), zhi)) : z2;
+                    int o0, o1;
+                    float2 F, x0, x1;
+                    if (TEX8) {
+                        const float2 m = add2_rd(fma2_rd(zs, f2(256.f), f2(-127.5f)), f2(12582912.f));
+                        const int b0 = __float_as_int(m.x), b1 = __float_as_int(m.y);
+                        o0 = (b0 >> 8) + r0;
+                        o1 = (b1 >> 8) + r1;
+                        // Fr = 2^23 + F, F the fast weight (0..255)
+                        const float2 Fr =
+                            f2(__int_as_float((b0 & 255) | 0x4B000000), __int_as_float((b1 & 255) | 0x4B000000));
+                        F = add2(Fr, f2(-8388608.f));
+                        // x1 = floor(F S / 256 + 1/2), all steps exact
+                        x1 = add2(add2_rd(fma2(F, S256, f2(0.5f)), f2(12582912.f)), f2(-12582912.f));
+                        if (RULE == 1)  // F + floor(1/2 - F S / 256); Fr - 2.5 * 2^23 = F - 1.5 * 2^23
+                            x0 = add2(add2_rd(fma2(F, f2(-S256.x, -S256.y), f2(0.5f)), f2(12582912.f)),
+                                      add2(Fr, f2(-20971520.f)));
+                        else
+                            x0 = sub2(F, x1);
+                    } else {
+                        const float2 xb = add2(zs, f2(-0.5f)), m = add2_rd(xb, f2(12582912.f));
+                        o0 = __float_as_int(m.x) + r0;
+                        o1 = __float_as_int(m.y) + r1;
+                        F = sub2(xb, add2(m, f2(-12582912.f)));
+                        x1 = mul2(F, S);
+                        x0 = sub2(F, x1);
+                    }
+                    const float2 t00 = f2(ld(vol + o0), ld(vol + o1));
+                    const float2 t10 = f2(ld(vol + o0 + 1), ld(vol + o1 + 1));
+                    const float2 t01 = f2(ld(vol1 + o0), ld(vol1 + o1));
+                    const float2 t11 = f2(ld(vol1 + o0 + 1), ld(vol1 + o1 + 1));
+                    v2 = TEX8 ? fma2(f2(256.f), t00, v2) : add2(v2, t00);
+                    v2 = fma2(S, sub2(t01, t00), v2);
+                    v2 = fma2(x1, sub2(t11, t01), v2);
+                    v2 = fma2(x0, sub2(t10, t00), v2);
+                    z2 = add2(z2, a2);
+                    if (PATH == 2)
+                        y2.x = __fadd_rn(y2.x, a1.x);
+                    else
+                        y2 = add2(y2, a1);
+                }
+                val[0] = v2.x;
+                val[FP_RPT - 1] = v2.y;
+            };
+            if (all_in)
+                pair_loop(std::false_type{});
+            else if constexpr (PAD)
+                pair_loop(std::true_type{});
         } else if (all_in) {
 #pragma unroll FP_UNROLL
             for (int sl = off; sl < end; ++sl) {
@@ -369,7 +475,8 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
 // in 32 bits), whose shared-D1 rays trace mixed slabs with the clamped
 // paired loop; a separate kernel with its own register budget keeps the
 // other kernels' allocation as it was.
-template <typename TV, typename TP, bool TEX8, int EPI, bool SUMS = false, bool PAD = false>
+// GENERAL: and the one whose other CUDA-core rays are paired as well.
+template <typename TV, typename TP, bool TEX8, int EPI, bool SUMS = false, bool PAD = false, bool GENERAL = false>
 __device__ __forceinline__ void fp_block(const FpArgs& L, int t) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ct = t % L.col_tiles;
@@ -398,14 +505,14 @@ __device__ __forceinline__ void fp_block(const FpArgs& L, int t) {
         fp_trace<TV, TP, TEX8, EPI, 3, 0, true, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
     else if (use_tex)
         fp_trace<TV, TP, TEX8, EPI, 3, 0, false, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
-    else if (shared && rule == 1)
+    else if (TEX8 && shared && rule == 1)
         fp_trace<TV, TP, TEX8, EPI, 2, 1, false, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
     else if (shared)
         fp_trace<TV, TP, TEX8, EPI, 2, 0, false, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
-    else if (fast && rule == 1)
-        fp_trace<TV, TP, TEX8, EPI, 1, 1, false, SUMS>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+    else if (TEX8 && fast && rule == 1)
+        fp_trace<TV, TP, TEX8, EPI, 1, 1, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
     else if (fast)
-        fp_trace<TV, TP, TEX8, EPI, 1, 0, false, SUMS>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 1, 0, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
     else
         fp_trace<TV, TP, TEX8, EPI, 0, 0, false, SUMS>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
 }
@@ -415,10 +522,12 @@ __global__ void __launch_bounds__(32 * FP_COLS, KK_FP_MINBLOCKS) cone_fp_kernel(
     fp_block<TV, TP, TEX8, EPI, SUMS>(L, blockIdx.x);
 }
 
-// cone_fp_kernel on a zero-padded volume copy (texture-compatible weights)
-template <typename TV, typename TP, int EPI>
-__global__ void __launch_bounds__(32 * FP_COLS, KK_FP_PAD_MINBLOCKS) cone_fp_pad_kernel(const FpArgs L) {
-    fp_block<TV, TP, true, EPI, false, true>(L, blockIdx.x);
+// cone_fp_kernel on a zero-padded volume copy
+template <typename TV, typename TP, bool TEX8, int EPI, bool GENERAL>
+__global__ void __launch_bounds__(32 * FP_COLS, GENERAL ? KK_FP_GENERAL_MINBLOCKS
+                                                : TEX8  ? KK_FP_PAD_MINBLOCKS
+                                                        : KK_FP_EXACT_MINBLOCKS) cone_fp_pad_kernel(const FpArgs L) {
+    fp_block<TV, TP, TEX8, EPI, false, true, GENERAL>(L, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -876,6 +985,7 @@ static bool brick_prepare(FpBrick& B, const FpArgs& L) {
 struct FpLaunch {
     int span_setting;    // as kk_fp_options.span
     bool tiles;          // shared-memory tiles where the rays qualify
+    bool general;        // KK_FP_OPT_GENERAL
     float* sums;         // float32 running sums for 16-bit outputs, or NULL
     int64_t sums_elems;  // its size in elements
 };
@@ -917,6 +1027,19 @@ static bool launch_fp_sums(const FpArgs& base, bool tex8, cudaStream_t s, const 
 }
 
 template <typename TV, typename TP, int EPI>
+static void launch_fp_padded(const FpArgs& L, bool tex8, bool general, unsigned blocks, cudaStream_t s) {
+    const int threads = 32 * FP_COLS;
+    if (tex8 && general)
+        cone_fp_pad_kernel<TV, TP, true, EPI, true><<<blocks, threads, 0, s>>>(L);
+    else if (tex8)
+        cone_fp_pad_kernel<TV, TP, true, EPI, false><<<blocks, threads, 0, s>>>(L);
+    else if (general)
+        cone_fp_pad_kernel<TV, TP, false, EPI, true><<<blocks, threads, 0, s>>>(L);
+    else
+        cone_fp_pad_kernel<TV, TP, false, EPI, false><<<blocks, threads, 0, s>>>(L);
+}
+
+template <typename TV, typename TP, int EPI>
 static void launch_fp_typed(const FpArgs& base, bool tex8, cudaStream_t s, const FpLaunch& opt) {
     if (!std::is_same<TP, float>::value && launch_fp_sums<TV, TP, EPI>(base, tex8, s, opt)) return;
     FpArgs L = base;
@@ -945,8 +1068,8 @@ static void launch_fp_typed(const FpArgs& base, bool tex8, cudaStream_t s, const
         if (brick) {
             Bl.L = L;
             cone_fp_brick_kernel<EPI><<<(unsigned)blocks, 32 * BRICK_WARPS, BRICK_SMEM, s>>>(Bl);
-        } else if (tex8 && L.padded) {
-            cone_fp_pad_kernel<TV, TP, EPI><<<(unsigned)blocks, 32 * FP_COLS, 0, s>>>(L);
+        } else if (L.padded) {
+            launch_fp_padded<TV, TP, EPI>(L, tex8, opt.general, (unsigned)blocks, s);
         } else if (tex8) {
             cone_fp_kernel<TV, TP, true, EPI><<<(unsigned)blocks, 32 * FP_COLS, 0, s>>>(L);
         } else {
@@ -1120,14 +1243,15 @@ extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, c
             return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: texture and volume storage differ", who);
         L.vtex = vtex->tex;
     }
-    if (opts->padded && tex8 && !(opts->flags & KK_FP_OPT_TILES)) {
+    if (opts->padded && !(opts->flags & KK_FP_OPT_TILES)) {
         rc = fp_pad_volume(L, vol, opts, (cudaStream_t)stream, who);
         if (rc) return rc;
     }
     L.additive = opts->additive ? 1 : 0;
     if (opts->sums_elems < 0 || (opts->sums_elems > 0 && !opts->sums))
         return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: bad running-sum buffer", who);
-    const FpLaunch lo = {opts->span, (opts->flags & KK_FP_OPT_TILES) != 0, opts->sums, opts->sums_elems};
+    const FpLaunch lo = {opts->span, (opts->flags & KK_FP_OPT_TILES) != 0, (opts->flags & KK_FP_OPT_GENERAL) != 0,
+                         opts->sums, opts->sums_elems};
     if (opts->residual) {
         const kk_fp_residual* res = opts->residual;
         if (!res->y || !res->weight) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: residual operands are NULL", who);

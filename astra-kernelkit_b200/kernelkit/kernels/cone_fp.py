@@ -130,10 +130,10 @@ class RayDrivenConeFP(BaseKernel):
     #: traced in chunks that fit it); 0 traces 16-bit projections in one
     #: launch
     sums_bytes = 1 << 30
-    #: texture-compatible weights: trace from a copy of the volume with two
-    #: zero texels around every axis, made at the start of every call
-    #: (same results; the CUDA-core rays of circular scans then sample the
-    #: slabs that cross the volume's boundary without per-texel tests)
+    #: trace from a copy of the volume with two zero texels around every
+    #: axis, made at the start of every call (the CUDA-core rays then sample
+    #: in pairs, the slabs that cross the volume's boundary without
+    #: per-texel tests; same results, with exact weights up to rounding)
     padded_copy = True
 
     def __init__(self, pixels_per_block: tuple = None,
@@ -170,6 +170,7 @@ class RayDrivenConeFP(BaseKernel):
         self.interpolation = interpolation
         self._params_dev = None
         self._n_params = 0
+        self._general = False
         self._axes_known = False
 
     @property
@@ -276,6 +277,12 @@ class RayDrivenConeFP(BaseKernel):
             # records without a texture path)
             core = np.floor((pos + 1) * f) > np.floor(pos * f)
             rec["flags"][sel] = np.where(core, _native.KK_FP_NO_TEXTURE, 0)
+        # circular scans: v has no component along the ray axis and the
+        # first in-slice axis, so a column's rows share that coordinate
+        n = np.arange(len(rec))
+        first = np.where(rec["axis"] == 1, 0, 1)
+        self._general = bool(np.any(rec["v"][n, rec["axis"]])
+                             or np.any(rec["v"][n, first]))
         order = np.argsort(key, kind="stable")
         t = _arrays.torch()
         self._params_dev = t.from_numpy(
@@ -423,18 +430,23 @@ class RayDrivenConeFP(BaseKernel):
     def _padded(self, vdesc):
         """(pointer, elements) of the zero-padded volume copy's buffer,
         allocated once per projector, device, volume shape and type."""
-        if not self.padded_copy or self._interp != _native.KK_INTERP_TEX8:
+        if not self.padded_copy:
             return None, 0
         t = _arrays.torch()
         dt = {_native.KK_F32: t.float32, _native.KK_BF16: t.bfloat16,
               _native.KK_F16: t.float16}[int(vdesc.dtype)]
         n = int(np.prod([int(x) + 4 for x in vdesc.shape]))
+        if n >= 2 ** 31 - 0x4B4000 - 2:  # the kernels' 32-bit offsets
+            return None, 0
         buf = getattr(self, "_pad_buf", None)
         dev = t.cuda.current_device()
         if (buf is None or buf.numel() != n or buf.dtype != dt
                 or buf.device.index != dev):
             self._pad_buf = None
-            buf = t.empty(n, dtype=dt, device="cuda")
+            try:
+                buf = t.empty(n, dtype=dt, device="cuda")
+            except t.cuda.OutOfMemoryError:  # trace the volume itself
+                return None, 0
             self._pad_buf = buf
         return buf.data_ptr(), buf.numel()
 
@@ -450,7 +462,8 @@ class RayDrivenConeFP(BaseKernel):
         o.additive = int(bool(additive))
         o.span = int(_DEFAULT_SPAN if self.slices_per_launch is None
                      else self.slices_per_launch)
-        o.flags = _native.KK_FP_OPT_TILES if self.use_tiles else 0
+        o.flags = ((_native.KK_FP_OPT_TILES if self.use_tiles else 0)
+                   | (_native.KK_FP_OPT_GENERAL if self._general else 0))
         o.vtex = None if lay is None else lay.handle
         o.residual = (None if residual is None
                       else ctypes.cast(ctypes.pointer(residual),
