@@ -65,6 +65,10 @@ struct FpArgs {
     // vol is the interior of a copy with two zero texels before and after
     // every axis (the border rule as memory)
     int padded;
+    // column pairs: the blocks from full_blocks on trace the last row tile,
+    // of at most 32 rows, with the thread's two rays in two columns;
+    // pair_tiles column tiles of 2 FP_COLS (0: no such blocks)
+    int pair_tiles, full_blocks;
 };
 
 struct BpArgs {

@@ -40,6 +40,9 @@ namespace kk {
 #ifndef KK_FP_PAD_MINBLOCKS
 #define KK_FP_PAD_MINBLOCKS (40 / KK_FP_COLS)  // the padded-copy kernel: 48 registers, no spills
 #endif
+#ifndef KK_FP_PAIR_ROWS
+#define KK_FP_PAIR_ROWS 640  // most detector rows traced with column pairs (fp_blocks)
+#endif
 #ifndef KK_FP_GENERAL_MINBLOCKS
 #define KK_FP_GENERAL_MINBLOCKS (36 / KK_FP_COLS)
 #endif
@@ -132,9 +135,13 @@ __device__ __forceinline__ int span_class(float c0, float c1, int n) {
 }
 
 template <typename TV, typename TP, bool TEX8, int EPI, int PATH, int RULE, bool AF = false, bool SUMS = false,
-          bool PAD = false, bool PAIR1 = false>
+          bool PAD = false, bool GENERAL = false>
 __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, int rec, int a, int A, int D1, int D2,
-                                         int rule, bool a_fast, int r0, int c, int lane) {
+                                         int rule, bool a_fast, int r0, int c, int lane, bool cols2) {
+    // ray k of the thread: 32 rows further down, or FP_COLS columns on
+    auto row = [&](int k) { return r0 + lane + (GENERAL && cols2 ? 0 : 32 * k); };
+    auto col = [&](int k) { return c + (GENERAL && cols2 ? FP_COLS * k : 0); };
+    auto on_detector = [&](int k) { return row(k) < L.rows && (!GENERAL || col(k) < L.cols); };
     float src[3], cor[3], u[3], v[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -150,22 +157,21 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
     const float half1 = 0.5f * (float)n1, half2 = 0.5f * (float)n2;
     const float unit_inv = 1.f / weight_unit<TEX8>();
 
-    // output element of ray k (row r0 + lane + 32 k)
+    // output element of ray k
     auto out_ptr = [&](int k) -> TP* {
-        const int64_t off = (int64_t)(r0 + lane + 32 * k) * L.ps[1] + (int64_t)c * L.ps[2];
+        const int64_t off = (int64_t)row(k) * L.ps[1] + (int64_t)col(k) * L.ps[2];
         return L.table ? (TP*)L.table[a] + off : (TP*)L.out + (int64_t)a * L.ps[0] + off;
     };
     // running float32 sum of ray k between launches (16-bit outputs)
     auto sum_ptr = [&](int k) -> float* {
-        return L.sums + ((int64_t)rec * L.rows + (r0 + lane + 32 * k)) * L.cols + c;
+        return L.sums + ((int64_t)rec * L.rows + row(k)) * L.cols + col(k);
     };
     RaySetup R[FP_RPT];
     float acc[FP_RPT];
 #pragma unroll
     for (int k = 0; k < FP_RPT; ++k) {
-        const int r = r0 + lane + 32 * k;
-        const bool valid = r < L.rows;
-        R[k] = ray_setup(src, cor, u, v, A, D1, D2, valid ? r : 0, c, sc1, sc2);
+        const bool valid = on_detector(k);
+        R[k] = ray_setup(src, cor, u, v, A, D1, D2, valid ? row(k) : 0, !GENERAL || valid ? col(k) : c, sc1, sc2);
         acc[k] = !valid ? 0.f : (SUMS && L.load_sums) ? *sum_ptr(k) : L.additive ? ld_rw(out_ptr(k)) : 0.f;
     }
 
@@ -305,7 +311,7 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
                 shared_loop(std::false_type{});
             else if constexpr (PAD)
                 shared_loop(std::true_type{});
-        } else if (FP_RPT == 2 && PAD && (PATH == 2 || (PATH == 1 && PAIR1))) {
+        } else if (FP_RPT == 2 && PAD && (PATH == 2 || (PATH == 1 && GENERAL))) {
             // The same for exact weights (floor by rounding down at 2^23)
             // and for rays with D1 coordinates of their own (PATH 1), whose
             // D1 splits are paired too.
@@ -456,15 +462,14 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
 
 #pragma unroll
     for (int k = 0; k < FP_RPT; ++k) {
-        if (r0 + lane + 32 * k >= L.rows) continue;
+        if (!on_detector(k)) continue;
         if (SUMS && L.store_sums) {
             *sum_ptr(k) = acc[k];
             continue;
         }
         float out = acc[k];
         if (EPI == FP_RESIDUAL && L.final_pass) {
-            const int r = r0 + lane + 32 * k;
-            const int64_t e = (int64_t)a * L.ps[0] + (int64_t)r * L.ps[1] + (int64_t)c * L.ps[2];
+            const int64_t e = (int64_t)a * L.ps[0] + (int64_t)row(k) * L.ps[1] + (int64_t)col(k) * L.ps[2];
             out = __fmul_rn(__fsub_rn(out, ld((const TP*)L.res_y + e)), ld((const TP*)L.res_w + e));
         }
         st(out_ptr(k), out);
@@ -479,11 +484,14 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
 template <typename TV, typename TP, bool TEX8, int EPI, bool SUMS = false, bool PAD = false, bool GENERAL = false>
 __device__ __forceinline__ void fp_block(const FpArgs& L, int t) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ct = t % L.col_tiles;
-    t /= L.col_tiles;
+    const bool cols2 = GENERAL && L.pair_tiles && t >= L.full_blocks;
+    const int tiles = cols2 ? L.pair_tiles : L.col_tiles;
+    if (cols2) t -= L.full_blocks;
+    const int ct = t % tiles;
+    t /= tiles;
     const int rec = t % L.n_angles;
-    const int rt = t / L.n_angles;
-    const int c = ct * FP_COLS + warp;
+    const int rt = cols2 ? (L.rows - 1) / FP_ROWS_T : t / L.n_angles;
+    const int c = ct * (cols2 ? 2 : 1) * FP_COLS + warp;
     if (c >= L.cols) return;  // whole warp; the kernel has no block barrier
 
     const kk_fp_angle* P = L.angles + rec;
@@ -496,25 +504,26 @@ __device__ __forceinline__ void fp_block(const FpArgs& L, int t) {
     const int rule = 2 - L.rank[A];
     const bool a_fast = L.rank[D1] < L.rank[D2];
     const bool fast = L.vs[D2] == 1 && rule < 2;
-    const bool shared = fast && __ldg(&P->v[A]) == 0.f && __ldg(&P->v[D1]) == 0.f;
+    // (two columns have D1 coordinates of their own)
+    const bool shared = fast && !cols2 && __ldg(&P->v[A]) == 0.f && __ldg(&P->v[D1]) == 0.f;
     const int r0 = rt * FP_ROWS_T;
     // records flagged KK_FP_NO_TEXTURE run on the CUDA cores even when the
     // layered texture is given, so both units share the work
     const bool use_tex = L.vtex && L.rank[A] == 2 && !(__ldg(&P->flags) & KK_FP_NO_TEXTURE);
     if (use_tex && a_fast)
-        fp_trace<TV, TP, TEX8, EPI, 3, 0, true, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 3, 0, true, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
     else if (use_tex)
-        fp_trace<TV, TP, TEX8, EPI, 3, 0, false, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 3, 0, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
     else if (TEX8 && shared && rule == 1)
-        fp_trace<TV, TP, TEX8, EPI, 2, 1, false, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 2, 1, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
     else if (shared)
-        fp_trace<TV, TP, TEX8, EPI, 2, 0, false, SUMS, PAD>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 2, 0, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
     else if (TEX8 && fast && rule == 1)
-        fp_trace<TV, TP, TEX8, EPI, 1, 1, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 1, 1, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
     else if (fast)
-        fp_trace<TV, TP, TEX8, EPI, 1, 0, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 1, 0, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
     else
-        fp_trace<TV, TP, TEX8, EPI, 0, 0, false, SUMS>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane);
+        fp_trace<TV, TP, TEX8, EPI, 0, 0, false, SUMS, false, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
 }
 
 template <typename TV, typename TP, bool TEX8, int EPI, bool SUMS = false>
@@ -907,8 +916,9 @@ struct FpBatch {
     FpArgs p[KK_MAX_BATCH];
 };
 
-template <bool TEX8, int EPI>
-__global__ void __launch_bounds__(32 * FP_COLS, 32 / FP_COLS) cone_fp_batched_kernel(const __grid_constant__ FpBatch B) {
+template <bool TEX8, int EPI, bool PAD>
+__global__ void __launch_bounds__(32 * FP_COLS, 32 / FP_COLS)
+    cone_fp_batched_kernel(const __grid_constant__ FpBatch B) {
     __shared__ FpArgs Ls;
     const int b = blockIdx.x;
     int i = 0;
@@ -917,7 +927,7 @@ __global__ void __launch_bounds__(32 * FP_COLS, 32 / FP_COLS) cone_fp_batched_ke
     const int* src = reinterpret_cast<const int*>(&B.p[i]);
     for (int k = threadIdx.x; k < (int)(sizeof(FpArgs) / 4); k += blockDim.x) reinterpret_cast<int*>(&Ls)[k] = src[k];
     __syncthreads();
-    fp_block<float, float, TEX8, EPI>(Ls, b - B.block_start[i]);
+    fp_block<float, float, TEX8, EPI, false, PAD, PAD>(Ls, b - B.block_start[i]);
 }
 
 
@@ -1026,6 +1036,25 @@ static bool launch_fp_sums(const FpArgs& base, bool tex8, cudaStream_t s, const 
     return true;
 }
 
+// Column tiles and blocks of a launch (< 2^31: checked by the caller). A
+// last row tile of at most 32 rows would leave every thread's second ray
+// idle; the kernels that pair any two rays trace it two columns per thread
+// instead, at the price of their D1 splits and registers (ms without and
+// with: 64^3 x 96 rows 0.162 / 0.157, 128 x 128 x 100 x 150 rows 0.704 /
+// 0.635, 192^3 x 288 rows 3.12 / 2.92, 277^3 x 416 rows 12.07 / 11.62, 362^3
+// x 544 rows 31.2 / 30.3). The idle share falls with the rows: beyond
+// KK_FP_PAIR_ROWS circular scans keep their kernel.
+static int64_t fp_blocks(FpArgs& L, bool pairs) {
+    L.col_tiles = (L.cols + FP_COLS - 1) / FP_COLS;
+    const int64_t row_tiles = (L.rows + FP_ROWS_T - 1) / FP_ROWS_T, per = (int64_t)L.n_angles * L.col_tiles;
+    const int tail = L.rows % FP_ROWS_T;
+    L.pair_tiles = 0;
+    if (!pairs || tail == 0 || tail > 32) return row_tiles * per;
+    L.pair_tiles = (L.cols + 2 * FP_COLS - 1) / (2 * FP_COLS);
+    L.full_blocks = (int)((row_tiles - 1) * per);
+    return L.full_blocks + (int64_t)L.n_angles * L.pair_tiles;
+}
+
 template <typename TV, typename TP, int EPI>
 static void launch_fp_padded(const FpArgs& L, bool tex8, bool general, unsigned blocks, cudaStream_t s) {
     const int threads = 32 * FP_COLS;
@@ -1043,9 +1072,9 @@ template <typename TV, typename TP, int EPI>
 static void launch_fp_typed(const FpArgs& base, bool tex8, cudaStream_t s, const FpLaunch& opt) {
     if (!std::is_same<TP, float>::value && launch_fp_sums<TV, TP, EPI>(base, tex8, s, opt)) return;
     FpArgs L = base;
-    L.col_tiles = (L.cols + FP_COLS - 1) / FP_COLS;
-    const int row_tiles = (L.rows + FP_ROWS_T - 1) / FP_ROWS_T;
-    const int64_t blocks = (int64_t)row_tiles * L.n_angles * L.col_tiles;  // < 2^31: checked by the caller
+    const int tail = L.rows % FP_ROWS_T;
+    const bool pairs = L.padded && tail > 0 && tail <= 32 && L.rows <= KK_FP_PAIR_ROWS;
+    const int64_t blocks = fp_blocks(L, L.padded && (pairs || opt.general));
     const int nmax = max(L.vn[0], max(L.vn[1], L.vn[2]));
     // intermediate sums must stay float32: spans only for float32 output;
     // and a residual computed in place (out is y or the weight) needs its
@@ -1069,7 +1098,7 @@ static void launch_fp_typed(const FpArgs& base, bool tex8, cudaStream_t s, const
             Bl.L = L;
             cone_fp_brick_kernel<EPI><<<(unsigned)blocks, 32 * BRICK_WARPS, BRICK_SMEM, s>>>(Bl);
         } else if (L.padded) {
-            launch_fp_padded<TV, TP, EPI>(L, tex8, opt.general, (unsigned)blocks, s);
+            launch_fp_padded<TV, TP, EPI>(L, tex8, opt.general || pairs, (unsigned)blocks, s);
         } else if (tex8) {
             cone_fp_kernel<TV, TP, true, EPI><<<(unsigned)blocks, 32 * FP_COLS, 0, s>>>(L);
         } else {
@@ -1125,7 +1154,7 @@ __global__ void fp_pad_kernel(const T* __restrict__ src, T* __restrict__ dst, in
 // paired loops need every offset from the interior, within
 // [-interior, total - interior), in 32 bits: larger volumes keep tracing
 // the volume itself.
-static int fp_pad_volume(FpArgs& L, const kk_volume* vol, const kk_fp_options* opts, cudaStream_t s,
+static int fp_pad_volume(FpArgs& L, const kk_volume* vol, void* padded, int64_t padded_elems, cudaStream_t s,
                          const char* who) {
     int64_t n[3], st[3];
     for (int k = 0; k < 3; ++k) {
@@ -1134,20 +1163,20 @@ static int fp_pad_volume(FpArgs& L, const kk_volume* vol, const kk_fp_options* o
     }
     const int64_t pst[3] = {1, n[0] + 4, (n[0] + 4) * (n[1] + 4)};
     const int64_t total = pst[2] * (n[2] + 4);
-    if (opts->padded_elems < total)
+    if (padded_elems < total)
         return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: the padded copy needs %lld elements", who, (long long)total);
     if (total >= ((int64_t)1 << 31) - 0x4B4000 - 2) return KK_OK;
     const dim3 block(128, 4), grid((unsigned)((n[1] + 4 + 3) / 4), (unsigned)(n[2] + 4));
     const int es = vol->dtype == KK_F32 ? 4 : 2;
     if (es == 4)
-        fp_pad_kernel<float><<<grid, block, 0, s>>>((const float*)vol->data, (float*)opts->padded, (int)n[0],
+        fp_pad_kernel<float><<<grid, block, 0, s>>>((const float*)vol->data, (float*)padded, (int)n[0],
                                                    (int)n[1], (int)n[2], st[0], st[1], st[2]);
     else
         fp_pad_kernel<unsigned short><<<grid, block, 0, s>>>((const unsigned short*)vol->data,
-                                                           (unsigned short*)opts->padded, (int)n[0], (int)n[1],
+                                                           (unsigned short*)padded, (int)n[0], (int)n[1],
                                                            (int)n[2], st[0], st[1], st[2]);
     const int64_t interior = 2 * (pst[0] + pst[1] + pst[2]);
-    L.vol = (const char*)opts->padded + interior * es;
+    L.vol = (const char*)padded + interior * es;
     for (int k = 0; k < 3; ++k) L.vs[k] = pst[L.rank[k]];
     L.off32 = 1;
     L.padded = 1;
@@ -1244,7 +1273,7 @@ extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, c
         L.vtex = vtex->tex;
     }
     if (opts->padded && !(opts->flags & KK_FP_OPT_TILES)) {
-        rc = fp_pad_volume(L, vol, opts, (cudaStream_t)stream, who);
+        rc = fp_pad_volume(L, vol, opts->padded, opts->padded_elems, (cudaStream_t)stream, who);
         if (rc) return rc;
     }
     L.additive = opts->additive ? 1 : 0;
@@ -1341,7 +1370,25 @@ extern "C" int kk_cone_fp_layered(const kk_layered* vtex, const kk_volume* vol, 
     return kk_cone_fp_ex(vol, proj, angles, out_scale, &o, stream);
 }
 
+template <int EPI>
+static void launch_fp_batch(const FpBatch& B, bool tex8, bool pad, unsigned blocks, cudaStream_t s) {
+    const int threads = 32 * FP_COLS;
+    if (tex8 && pad)
+        cone_fp_batched_kernel<true, EPI, true><<<blocks, threads, 0, s>>>(B);
+    else if (tex8)
+        cone_fp_batched_kernel<true, EPI, false><<<blocks, threads, 0, s>>>(B);
+    else if (pad)
+        cone_fp_batched_kernel<false, EPI, true><<<blocks, threads, 0, s>>>(B);
+    else
+        cone_fp_batched_kernel<false, EPI, false><<<blocks, threads, 0, s>>>(B);
+}
+
 extern "C" int kk_cone_fp_batched(const kk_fp_problem* pr, int32_t n, int32_t interp, int32_t slab, void* stream) {
+    return kk_cone_fp_batched_ex(pr, n, interp, slab, nullptr, stream);
+}
+
+extern "C" int kk_cone_fp_batched_ex(const kk_fp_problem* pr, int32_t n, int32_t interp, int32_t slab,
+                                     const kk_fp_batch_options* opts, void* stream) {
     const char* who = "kk_cone_fp_batched";
     if (!pr || n < 1 || n > KK_MAX_BATCH)
         return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: need 1..%d problems, got %d", who, KK_MAX_BATCH, n);
@@ -1375,13 +1422,23 @@ extern "C" int kk_cone_fp_batched(const kk_fp_problem* pr, int32_t n, int32_t in
             L.res_w = q.residual.weight;
         }
         L.additive = q.additive ? 1 : 0;
-        L.col_tiles = (L.cols + FP_COLS - 1) / FP_COLS;
         // a residual computed in place needs its operand intact: one launch
         const bool in_place = res && (L.res_y == L.out || L.res_w == L.out);
         const int nmax = max(L.vn[0], max(L.vn[1], L.vn[2]));
         spans[i] = in_place ? 0 : fp_span(nmax, L.slab, q.span);
         passes[i] = spans[i] ? (nmax + spans[i] - 1) / spans[i] : 1;
         max_passes = max(max_passes, passes[i]);
+    }
+    // trace from zero-padded copies when every problem has a buffer (and
+    // offsets in 32 bits)
+    bool pad = opts && opts->padded;
+    for (int i = 0; pad && i < n; ++i) {
+        const int64_t* v = pr[i].vol.shape;
+        pad = opts->padded[i] && (v[0] + 4) * (v[1] + 4) * (v[2] + 4) < ((int64_t)1 << 31) - 0x4B4000 - 2;
+    }
+    for (int i = 0; pad && i < n; ++i) {
+        const int rc = fp_pad_volume(args[i], &pr[i].vol, opts->padded[i], opts->padded_elems[i], st, who);
+        if (rc) return rc;
     }
     // launch p traces span p of every problem that has one; plain and
     // residual problems are launched apart
@@ -1399,7 +1456,7 @@ extern "C" int kk_cone_fp_batched(const kk_fp_problem* pr, int32_t n, int32_t in
                     L.additive = p == 0 ? args[i].additive : 1;
                     L.final_pass = p == passes[i] - 1;
                 }
-                const int64_t blocks = (int64_t)((L.rows + FP_ROWS_T - 1) / FP_ROWS_T) * L.n_angles * L.col_tiles;
+                const int64_t blocks = fp_blocks(L, pad);
                 B.p[B.n] = L;
                 B.block_start[B.n] = (int)total;
                 total += blocks;
@@ -1409,18 +1466,10 @@ extern "C" int kk_cone_fp_batched(const kk_fp_problem* pr, int32_t n, int32_t in
             }
             if (B.n == 0) continue;
             B.block_start[B.n] = (int)total;
-            const bool tex8 = interp == KK_INTERP_TEX8;
-            if (kind == 0) {
-                if (tex8)
-                    cone_fp_batched_kernel<true, FP_STORE><<<(unsigned)total, 32 * FP_COLS, 0, st>>>(B);
-                else
-                    cone_fp_batched_kernel<false, FP_STORE><<<(unsigned)total, 32 * FP_COLS, 0, st>>>(B);
-            } else {
-                if (tex8)
-                    cone_fp_batched_kernel<true, FP_RESIDUAL><<<(unsigned)total, 32 * FP_COLS, 0, st>>>(B);
-                else
-                    cone_fp_batched_kernel<false, FP_RESIDUAL><<<(unsigned)total, 32 * FP_COLS, 0, st>>>(B);
-            }
+            if (kind == 0)
+                launch_fp_batch<FP_STORE>(B, interp == KK_INTERP_TEX8, pad, (unsigned)total, st);
+            else
+                launch_fp_batch<FP_RESIDUAL>(B, interp == KK_INTERP_TEX8, pad, (unsigned)total, st);
             const int rc = kk_check_launch(who);
             if (rc) return rc;
         }

@@ -78,6 +78,11 @@ class kk_fp_problem(ctypes.Structure):
                 ("span", ctypes.c_int32)]
 
 
+class kk_fp_batch_options(ctypes.Structure):
+    _fields_ = [("padded", ctypes.POINTER(ctypes.c_void_p)),
+                ("padded_elems", ctypes.POINTER(ctypes.c_int64))]
+
+
 class kk_bp_problem(ctypes.Structure):
     _fields_ = [("tex", ctypes.c_void_p), ("vol", kk_volume),
                 ("angles", ctypes.c_void_p), ("out_scale", ctypes.c_float),
@@ -111,6 +116,7 @@ EXPORTS = ("kk_cone_fp_ex", "kk_fp_launches_ex", "kk_wait_timeouts",
            "kk_cone_bp_layered_batched_ex", "kk_bp_batch_sync_elems",
            "kk_cone_fp", "kk_cone_fp_residual", "kk_cone_fp_layered",
            "kk_cone_fp_adjoint", "kk_cone_fp_batched",
+           "kk_cone_fp_batched_ex",
            "kk_cone_bp_layered_batched",
            "kk_cone_bp", "kk_cone_bp_static",
            "kk_cone_bp_update", "kk_layered_create", "kk_layered_copy",
@@ -156,6 +162,8 @@ def load():
     L.kk_cone_fp_adjoint.argtypes = [P(kk_projections), P(kk_volume), vp,
                                      vp, i32, i32, i32, vp, i64, vp]
     L.kk_cone_fp_batched.argtypes = [P(kk_fp_problem), i32, i32, i32, vp]
+    L.kk_cone_fp_batched_ex.argtypes = [P(kk_fp_problem), i32, i32, i32,
+                                        P(kk_fp_batch_options), vp]
     L.kk_cone_bp_layered_batched.argtypes = [P(kk_bp_problem), i32, vp]
     L.kk_cone_bp_layered_batched_ex.argtypes = [P(kk_bp_problem), i32,
                                                 P(kk_bp_batch_options), vp]

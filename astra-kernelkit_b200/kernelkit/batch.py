@@ -20,6 +20,7 @@ call (``algo.py:226-368``); each problem's arithmetic is the same as
 """
 from __future__ import annotations
 
+import ctypes
 import json
 import os
 from typing import Callable, Sequence
@@ -145,17 +146,24 @@ class BatchedSIRT:
         for g in range(0, n, _native.KK_MAX_BATCH):
             m = min(_native.KK_MAX_BATCH, n - g)
             fa = (_native.kk_fp_problem * m)(*self._fp[g:g + m])
+            # the projectors' zero-padded volume copies (used when all have
+            # one)
+            pads = [s.fp._padded(_native.volume_desc(s.x))
+                    for s in self.solvers[g:g + m]]
+            ptrs = (ctypes.c_void_p * m)(*[p for p, _ in pads])
+            elems = (ctypes.c_int64 * m)(*[e for _, e in pads])
+            fo = _native.kk_fp_batch_options(ptrs, elems)
             ba = (_native.kk_bp_problem * m)(*self._bp[g:g + m])
             opts = None
             if self.persistent:
-                elems = int(L.kk_bp_batch_sync_elems(ba, m))
-                if elems < 0:
+                n_sync = int(L.kk_bp_batch_sync_elems(ba, m))
+                if n_sync < 0:
                     _native.check(_native.KK_ERR_INVALID_ARGUMENT)
-                sync = t.zeros(elems, dtype=t.int32, device="cuda")
-                opts = _native.kk_bp_batch_options(1, sync.data_ptr(), elems,
-                                                   0, -1)
+                sync = t.zeros(n_sync, dtype=t.int32, device="cuda")
+                opts = _native.kk_bp_batch_options(1, sync.data_ptr(),
+                                                   n_sync, 0, -1)
                 opts._sync = sync  # keep the buffer alive with the options
-            self._fp_groups.append((fa, m))
+            self._fp_groups.append((fa, m, fo))
             self._bp_groups.append((ba, m, opts))
         self._graph = None
         self._t = t
@@ -212,9 +220,9 @@ class BatchedSIRT:
         for s, lay in zip(self.solvers, self._vtex):
             if lay is not None:
                 lay.copy_from(s.x)
-        for fa, m in self._fp_groups:
-            _native.check(L.kk_cone_fp_batched(
-                fa, m, _native.KK_INTERP_TEX8, 16, stream))
+        for fa, m, fo in self._fp_groups:
+            _native.check(L.kk_cone_fp_batched_ex(
+                fa, m, _native.KK_INTERP_TEX8, 16, fo, stream))
         for s in self.solvers:
             s.tex.copy_from(s.y_tmp)
         for ba, m, opts in self._bp_groups:
@@ -252,8 +260,6 @@ class BatchedSIRT:
 
 
 def ctypes_float9(a) -> object:
-    import ctypes
-
     return (ctypes.c_float * 9)(*[float(v) for v in np.asarray(a).reshape(9)])
 
 

@@ -388,6 +388,20 @@ KK_API int kk_cone_fp_batched(const kk_fp_problem* problems, int32_t n,
                               int32_t interp, int32_t slab, void* stream);
 
 typedef struct {
+    void* const* padded;         /* NULL, or n device buffers for the
+                                    problems' zero-padded volume copies
+                                    (as kk_fp_options.padded); used when
+                                    every problem has one */
+    const int64_t* padded_elems; /* their elements */
+} kk_fp_batch_options;
+
+/* kk_cone_fp_batched with options (NULL: none); same results. */
+KK_API int kk_cone_fp_batched_ex(const kk_fp_problem* problems, int32_t n,
+                                 int32_t interp, int32_t slab,
+                                 const kk_fp_batch_options* options,
+                                 void* stream);
+
+typedef struct {
     const kk_layered* tex;      /* the projections (kk_layered_copy) */
     kk_volume vol;              /* float32 */
     const kk_bp_angle* angles;

@@ -1,6 +1,7 @@
-"""Paired rays of the padded forward projector: exact weights, and detectors
-whose rows do not share their in-slice coordinate (tilted), against the
-unpadded projector, over ray directions, layouts, storage types, slice
+"""Paired rays of the padded forward projector: exact weights, detectors
+whose rows do not share their in-slice coordinate (tilted), and last row
+tiles of at most 32 rows (two columns per thread), against the unpadded
+projector, over ray directions, layouts, storage types, slice
 spans and extents that leave partial slabs, rows and columns. Texture-
 compatible weights agree bit for bit; exact weights up to the rounding of
 a product that only one of the two fuses."""
@@ -34,8 +35,9 @@ def _scan(kind, n=14, rows=70, cols=41):
             for k in range(n)]
 
 
-def _project(kind, interp, padded, vol, axes, span=None, tex=True):
-    pgs = _scan(kind)
+def _project(kind, interp, padded, vol, axes, span=None, tex=True, rows=70,
+             cols=41, residual=None):
+    pgs = _scan(kind, rows=rows, cols=cols)
     shape = [0, 0, 0]
     for k in range(3):
         shape[axes[k]] = vol.shape[k]
@@ -49,7 +51,10 @@ def _project(kind, interp, padded, vol, axes, span=None, tex=True):
     assert K._general == (kind != "circular")
     det = pgs[0].detector
     out = torch.zeros((len(pgs), det.rows, det.cols), device="cuda")
-    K(vol, pgs, vg, out, additive=False)
+    if residual is None:
+        K(vol, pgs, vg, out, additive=False)
+    else:
+        K.residual(vol, pgs, vg, out, *residual)
     assert float(out.abs().sum()) > 0
     return out
 
@@ -86,3 +91,69 @@ def test_padded_pairs_options(kind, interp):
     _same(kind, interp, vol[:, 1:, 2:37])
     _same(kind, interp, vol.to(torch.bfloat16))
     _same(kind, interp, vol.to(torch.float16))
+
+
+@pytest.mark.parametrize("kind", ["circular", "tilted", "alldirs"])
+@pytest.mark.parametrize("rows,cols", [(1, 9), (32, 8), (33, 12), (64, 5),
+                                       (65, 4), (96, 13), (640, 7),
+                                       (641, 7)])
+def test_last_row_tiles(rows, cols, kind):
+    vol = _volume((24, 26, 40))
+    for interp in ("texture", "exact"):
+        _same(kind, interp, vol, rows=rows, cols=cols)
+    y, w = (torch.rand((14, rows, cols), device="cuda") for _ in range(2))
+    _same(kind, "texture", vol, rows=rows, cols=cols, residual=(y, w),
+          span=16)
+
+
+def test_batched_padded_copies():
+    """kk_cone_fp_batched_ex from padded copies gives the unpadded launches'
+    projections bit for bit, and keeps to the volumes when one problem has
+    no copy."""
+    import ctypes
+
+    from kernelkit import _native
+
+    L = _native.load()
+    jobs = []
+    for n, rows, cols in ((21, 40, 30), (40, 70, 61), (33, 64, 9)):
+        pgs = _scan("circular", n=9, rows=rows, cols=cols)
+        vg = kk.resolve_volume_geometry(shape=n, voxel_size=1.0)
+        K = RayDrivenConeFP()
+        K.compile()
+        K.set_params(K.geoms2params(pgs, vg))
+        jobs.append((K, _volume((n, n, n)), (9, rows, cols), vg))
+
+    def run(options):
+        outs = [torch.zeros(s, device="cuda") for _, _, s, _ in jobs]
+        pr = (_native.kk_fp_problem * len(jobs))()
+        keep = []
+        for q, (K, vol, _, vg), out in zip(pr, jobs, outs):
+            q.vol = _native.volume_desc(vol)
+            q.proj = _native.projections_desc(out)
+            q.angles = K._params_dev.data_ptr()
+            q.out_scale[:] = [float(v) for r in K._output_scale(vg.voxel_size)
+                              for v in r]
+            lay = _native.Layered(*vol.shape, _native.KK_F32)
+            lay.copy_from(vol)
+            keep.append(lay)
+            q.vtex = lay.handle
+            q.span = 16
+        _native.check(L.kk_cone_fp_batched_ex(
+            pr, len(jobs), _native.KK_INTERP_TEX8, 16, options,
+            _native.current_stream()))
+        torch.cuda.synchronize()
+        return outs
+
+    def options(skip=None):
+        pads = [K._padded(_native.volume_desc(v)) for K, v, _, _ in jobs]
+        ptr = (ctypes.c_void_p * 3)(*[None if i == skip else p
+                                      for i, (p, _) in enumerate(pads)])
+        return _native.kk_fp_batch_options(
+            ptr, (ctypes.c_int64 * 3)(*[e for _, e in pads]))
+
+    ref = run(None)
+    assert all(float(r.abs().sum()) > 0 for r in ref)
+    for o in (options(), options(skip=1)):
+        for a, b in zip(run(o), ref):
+            assert torch.equal(a, b)
