@@ -3,11 +3,15 @@
 #include <algorithm>
 #include <mutex>
 
-#ifndef KK_BP_LANES
-#define KK_BP_LANES 1  // 2 x 2 quads of lanes (0: lanes along the fastest axis)
-#endif
 #ifndef KK_BP_WZ
 #define KK_BP_WZ 16  // voxels per warp along the fastest axis
+#endif
+
+#ifndef KK_BP_CHUNKS_PER_LAUNCH
+#define KK_BP_CHUNKS_PER_LAUNCH 4
+#endif
+#ifndef KK_BP_SPLIT_BLOCKS
+#define KK_BP_SPLIT_BLOCKS 40  // blocks per SM up to which launches are split (launch_bp_tex)
 #endif
 
 #include "kk_cone.cuh"
@@ -65,13 +69,13 @@ __device__ __forceinline__ float gather_exact(cudaTextureObject_t tex, float V, 
 // 1 % because the fetches bind): 90.2 -> 81.9 ms and 5.76 -> 5.38 ms, the
 // skipping alone 87.2 and 5.74. Per-warp boxes would miss 10.6 % but test
 // eight times as often.
+template <int TY>
 __device__ __forceinline__ unsigned bp_block_misses(const BpArgs& L, int j0, int nj, int bx, int by, int g0, int cnt,
                                                     int tid) {
     const int jj = tid >> 3, corner = tid & 7;
-    static_assert(BP_TILE_2 * BP_TILE_1 == 8 * BP_CHUNK, "eight corner threads per angle");
     const int n0 = L.vn[L.m0], n1 = L.vn[L.m1], n2 = L.vn[L.m2];
     const int c0 = (corner & 1) ? g0 + cnt - 1 : g0;
-    const int c1 = (corner & 2) ? min(by * BP_TILE_1 + BP_TILE_1, n1) - 1 : by * BP_TILE_1;
+    const int c1 = (corner & 2) ? min(by * TY + TY, n1) - 1 : by * TY;
     const int c2 = (corner & 4) ? min(bx * BP_TILE_2 + BP_TILE_2, n2) - 1 : bx * BP_TILE_2;
     const float p0 = (float)c0 - 0.5f * (float)n0 + 0.5f;
     const float p1 = (float)c1 - 0.5f * (float)n1 + 0.5f;
@@ -112,19 +116,22 @@ __device__ __forceinline__ unsigned bp_block_misses(const BpArgs& L, int j0, int
     return miss;
 }
 
-template <typename TP, typename TV, bool TEX8, int EPI, int FETCH>
+// TY: voxels per block along the middle axis. SPLIT: the block has a layer
+// of threads (threadIdx.z) per chunk of the launch, each accumulates its own
+// chunk, and the first adds the chunks' sums to the running sum in order.
+template <typename TP, typename TV, bool TEX8, int EPI, int FETCH, int TY = BP_TILE_1, bool SPLIT = false>
 __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz) {
     // One launch covers the angles [j_begin, j_end): one 32-angle chunk,
     // as one launch of the reference does (kernels/cone_bp.py:297-302), so
     // the chunk's projections stay in L2 while every voxel reads them; the
     // running sum vol += acc * scale is carried between launches in the
     // volume (float32) or in the float32 work buffer.
-    __shared__ kk_bp_angle sp[BP_CHUNK];
-    __shared__ unsigned char s_miss[BP_CHUNK / 4];  // per warp: four angles of bp_block_misses
-#if KK_BP_LANES == 0
-    const int i2 = bx * BP_TILE_2 + threadIdx.x;
-    const int i1 = by * BP_TILE_1 + threadIdx.y;
-#else
+    constexpr int LAYERS = SPLIT ? KK_BP_CHUNKS_PER_LAUNCH : 1, THREADS = BP_TILE_2 * TY;
+    __shared__ kk_bp_angle s_angles[LAYERS][BP_CHUNK];
+    __shared__ unsigned char s_missed[LAYERS][BP_CHUNK / 4];  // four angles of bp_block_misses each
+    const int layer = SPLIT ? threadIdx.z : 0;
+    kk_bp_angle* sp = s_angles[layer];
+    unsigned char* s_miss = s_missed[layer];
     // warps cover KK_BP_WZ (fastest axis) x 32 / KK_BP_WZ (middle axis)
     // voxels, and every quad of lanes a 2 x 2 square of them
     const int lane = threadIdx.x, w = threadIdx.y;
@@ -132,8 +139,7 @@ __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz
     const int zl = (lane & 1) | (((lane >> 2) * 2) % WZ);
     const int yl = ((lane >> 1) & 1) | ((((lane >> 2) * 2) / WZ) * 2);
     const int i2 = bx * BP_TILE_2 + (w % (BP_TILE_2 / WZ)) * WZ + zl;
-    const int i1 = by * BP_TILE_1 + (w / (BP_TILE_2 / WZ)) * WY + yl;
-#endif
+    const int i1 = by * TY + (w / (BP_TILE_2 / WZ)) * WY + yl;
     const int g0 = bz * BP_GROUP;
     const int n0 = L.vn[L.m0], n1 = L.vn[L.m1], n2 = L.vn[L.m2];
     const bool active = i2 < n2 && i1 < n1;
@@ -159,7 +165,7 @@ __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz
     for (int i = 0; i < BP_GROUP; ++i) {
         acc[i] = 0.f;
         vacc[i] = 0.f;
-        if (active && i < cnt) {
+        if (active && i < cnt && layer == 0) {
             if (L.load_mode == LOAD_VOL)
                 vacc[i] = L.fresh ? ld_cv(vol + vbase + i * vstep) : ld_cs(vol + vbase + i * vstep);
             else if (L.load_mode == LOAD_WORK)
@@ -168,19 +174,24 @@ __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz
     }
 
     const int tid = threadIdx.y * BP_TILE_2 + threadIdx.x;
-    for (int j0 = L.j_begin; j0 < L.j_end; j0 += BP_CHUNK) {
+    // (SPLIT: one round, as a launch has a chunk per layer)
+    for (int j0 = L.j_begin + layer * BP_CHUNK; SPLIT || j0 < L.j_end; j0 += BP_CHUNK) {
         const int nj = min(BP_CHUNK, L.j_end - j0);
         __syncthreads();
-        for (int k = tid; k < nj * 12; k += BP_TILE_2 * BP_TILE_1)
+        for (int k = tid; k < nj * 12; k += THREADS)
             ((float*)sp)[k] = __ldg((const float*)(L.angles + j0) + k);
-        const unsigned miss = bp_block_misses(L, j0, nj, bx, by, g0, cnt, tid);
-        if ((tid & 31) == 0) s_miss[tid >> 5] = (unsigned char)miss;
+#pragma unroll
+        for (int q = 0; q < BP_CHUNK; q += THREADS / 8) {
+            const unsigned miss = bp_block_misses<TY>(L, j0 + q, nj - q, bx, by, g0, cnt, tid);
+            if ((tid & 31) == 0) s_miss[(q >> 2) + (tid >> 5)] = (unsigned char)miss;
+        }
         __syncthreads();
-        if (!active) continue;
+        if (!SPLIT && !active) continue;
         // one bit per angle of the chunk that may reach the block
         unsigned live = nj == BP_CHUNK ? 0xffffffffu : (1u << nj) - 1u;
 #pragma unroll
         for (int k = 0; k < BP_CHUNK / 4; ++k) live &= ~((unsigned)s_miss[k] << (4 * k));
+        if (SPLIT && !active) live = 0;
         while (live) {
             const int jj = __ffs(live) - 1;
             live &= live - 1;
@@ -235,10 +246,28 @@ __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz
                 dn = __fadd_rn(dn, dd);
             }
         }
+        if constexpr (SPLIT) {
+            break;
+        } else {
+#pragma unroll
+            for (int i = 0; i < BP_GROUP; ++i) {
+                vacc[i] = fmaf(acc[i], L.scale, vacc[i]);
+                acc[i] = 0.f;
+            }
+        }
+    }
+    if (SPLIT) {
+        __shared__ float s_sums[LAYERS > 1 ? LAYERS - 1 : 1][BP_GROUP][THREADS];
+        if (layer > 0) {
+#pragma unroll
+            for (int i = 0; i < BP_GROUP; ++i) s_sums[layer - 1][i][tid] = acc[i];
+        }
+        __syncthreads();
+        if (layer > 0) return;
 #pragma unroll
         for (int i = 0; i < BP_GROUP; ++i) {
             vacc[i] = fmaf(acc[i], L.scale, vacc[i]);
-            acc[i] = 0.f;
+            for (int q = 1; q < (int)blockDim.z; ++q) vacc[i] = fmaf(s_sums[q - 1][i][tid], L.scale, vacc[i]);
         }
     }
     if (!active) return;
@@ -314,6 +343,19 @@ __global__ void layered_fill_kernel(const float* src, const uint64_t* table, int
     const float* p = (table ? (const float*)table[a] : src + (int64_t)a * sa) + (int64_t)c * sc;
     for (int r = blockIdx.y * 8; r < min(rows, (int)blockIdx.y * 8 + 8); ++r)
         surf2DLayeredwrite(__ldg(p + (int64_t)r * sr), surf, c * (int)sizeof(float), r, layer);
+}
+
+// cone_bp_kernel through the texture with a layer of threads per 32-angle
+// chunk (SPLIT), for volumes whose blocks do not fill the GPU: BP_SPLIT_1
+// voxels along the middle axis, so a block of four chunks has 256 threads.
+constexpr int BP_SPLIT_1 = 2;
+
+template <typename TV, int EPI>
+__global__ void __launch_bounds__(BP_TILE_2* BP_SPLIT_1* KK_BP_CHUNKS_PER_LAUNCH, 4) cone_bp_split_kernel(const BpArgs L) {
+    int bx, by, bz;
+    bp_tile_order(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), gridDim.x, gridDim.y, gridDim.z, bx,
+                  by, bz, KK_BP_TILE_Z, KK_BP_TILE_Y * (BP_TILE_1 / BP_SPLIT_1));
+    bp_block<float, TV, true, EPI, FETCH_TEX, BP_SPLIT_1, true>(L, bx, by, bz);
 }
 
 // Many problems in one launch (one 32-angle chunk of each): argument
@@ -464,6 +506,25 @@ static dim3 bp_grid(const BpArgs& L) {
                 (L.vn[L.m0] + BP_GROUP - 1) / BP_GROUP);
 }
 
+// One launch through the texture. Volumes of few blocks (four fit an SM)
+// are split by chunk: more and shorter blocks fill the GPU sooner and leave
+// a shorter last round (call times, 64^3 x 96 0.102 -> 0.088 ms, 128 x 128 x
+// 100 x 180 0.399 -> 0.381, 192 x 192 x 180 x 250, 31 blocks per SM, 1.643 ->
+// 1.628; 256^3 x 360, 74 per SM, 5.38 -> 5.52: the chunks' projections then
+// compete for L1). The running sum adds the chunks in the same order.
+template <typename TV, int EPI>
+static void launch_bp_tex(const BpArgs& L, cudaStream_t s) {
+    const dim3 g = bp_grid(L);
+    const int chunks = (L.j_end - L.j_begin + BP_CHUNK - 1) / BP_CHUNK;
+    const int64_t split_rows = (L.vn[L.m1] + BP_SPLIT_1 - 1) / BP_SPLIT_1;
+    if (chunks > 1 && chunks <= KK_BP_CHUNKS_PER_LAUNCH && split_rows <= MAX_GRID_Y &&
+        (int64_t)g.x * g.y * g.z <= (int64_t)kk_sm_count() * KK_BP_SPLIT_BLOCKS)
+        cone_bp_split_kernel<TV, EPI>
+            <<<dim3(g.x, (unsigned)split_rows, g.z), dim3(BP_TILE_2, BP_SPLIT_1, chunks), 0, s>>>(L);
+    else
+        cone_bp_kernel<float, TV, true, EPI, FETCH_TEX><<<g, dim3(BP_TILE_2, BP_TILE_1), 0, s>>>(L);
+}
+
 template <typename TP, typename TV, int EPI>
 static void launch_bp_typed(const BpArgs& L, bool tex8, cudaStream_t s) {
     dim3 block(BP_TILE_2, BP_TILE_1);
@@ -481,9 +542,6 @@ static void launch_bp_typed(const BpArgs& L, bool tex8, cudaStream_t s) {
 // those cases a single launch covers every angle (same arithmetic, more L2
 // traffic). Fewer launches save the running sum's round trip through
 // memory between chunks.
-#ifndef KK_BP_CHUNKS_PER_LAUNCH
-#define KK_BP_CHUNKS_PER_LAUNCH 4
-#endif
 constexpr int BP_LAUNCH_ANGLES = BP_CHUNK * KK_BP_CHUNKS_PER_LAUNCH;
 
 template <typename Fn>
@@ -754,11 +812,11 @@ extern "C" int kk_cone_bp_layered_ex(const kk_layered* t, int64_t n_angles, cons
         if (interp == KK_INTERP_EXACT)
             cone_bp_kernel<float, float, false, BP_STORE, FETCH_GATHER><<<bp_grid(c), block, 0, s>>>(c);
         else if (vdt == KK_F32)
-            cone_bp_kernel<float, float, true, BP_STORE, FETCH_TEX><<<bp_grid(c), block, 0, s>>>(c);
+            launch_bp_tex<float, BP_STORE>(c, s);
         else if (vdt == KK_BF16)
-            cone_bp_kernel<float, __nv_bfloat16, true, BP_STORE, FETCH_TEX><<<bp_grid(c), block, 0, s>>>(c);
+            launch_bp_tex<__nv_bfloat16, BP_STORE>(c, s);
         else
-            cone_bp_kernel<float, __half, true, BP_STORE, FETCH_TEX><<<bp_grid(c), block, 0, s>>>(c);
+            launch_bp_tex<__half, BP_STORE>(c, s);
     });
     return kk_check_launch(who);
 }
@@ -786,13 +844,12 @@ extern "C" int kk_cone_bp_layered_update(const kk_layered* t, const kk_volume* v
     const cudaStream_t s = (cudaStream_t)stream;
     const int vdt = vol->dtype;
     bp_chunks(L, vdt == KK_F32, false, true, [&](const BpArgs& c) {
-        const dim3 block(BP_TILE_2, BP_TILE_1);
         if (vdt == KK_F32)
-            cone_bp_kernel<float, float, true, BP_UPDATE, FETCH_TEX><<<bp_grid(c), block, 0, s>>>(c);
+            launch_bp_tex<float, BP_UPDATE>(c, s);
         else if (vdt == KK_BF16)
-            cone_bp_kernel<float, __nv_bfloat16, true, BP_UPDATE, FETCH_TEX><<<bp_grid(c), block, 0, s>>>(c);
+            launch_bp_tex<__nv_bfloat16, BP_UPDATE>(c, s);
         else
-            cone_bp_kernel<float, __half, true, BP_UPDATE, FETCH_TEX><<<bp_grid(c), block, 0, s>>>(c);
+            launch_bp_tex<__half, BP_UPDATE>(c, s);
     });
     return kk_check_launch(who);
 }
