@@ -722,6 +722,13 @@ extern "C" int kk_layered_destroy(kk_layered* t) {
     return KK_OK;
 }
 
+static void launch_layered_fill(kk_layered* t, const kk_projections* src, int64_t first, int64_t count,
+                                cudaStream_t s) {
+    const dim3 grid((unsigned)((src->cols + 127) / 128), (unsigned)((src->rows + 7) / 8), (unsigned)count);
+    layered_fill_kernel<<<grid, 128, 0, s>>>((const float*)src->data, src->table, src->stride[0], src->stride[1],
+                                             src->stride[2], (int)src->rows, (int)src->cols, (int)first, t->surf);
+}
+
 extern "C" int kk_layered_copy(kk_layered* t, const kk_projections* src, void* stream) {
     if (!t || !src) return kk_fail(KK_ERR_INVALID_ARGUMENT, "kk_layered_copy: NULL argument");
     if (src->table || !src->data)
@@ -764,9 +771,7 @@ extern "C" int kk_layered_fill(kk_layered* t, const kk_projections* src, int64_t
         if (e != cudaSuccess) return kk_fail(KK_ERR_CUDA, "%s: %s", who, cudaGetErrorString(e));
         return KK_OK;
     }
-    const dim3 grid((unsigned)((src->cols + 127) / 128), (unsigned)((src->rows + 7) / 8), (unsigned)count);
-    layered_fill_kernel<<<grid, 128, 0, s>>>((const float*)src->data, src->table, src->stride[0], src->stride[1],
-                                             src->stride[2], (int)src->rows, (int)src->cols, (int)first, t->surf);
+    launch_layered_fill(t, src, first, count, s);
     return kk_check_launch(who);
 }
 

@@ -17,7 +17,7 @@ def torch():
 
 def require_cuda():
     t = torch()
-    if not t.cuda.is_available():
+    if not (t.cuda.is_initialized() or t.cuda.is_available()):
         raise RuntimeError(
             "A CUDA device is required: the cone-beam projectors run only "
             "as CUDA kernels.")

@@ -246,7 +246,11 @@ def dtype_code(t) -> int:
 
 
 def current_stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(_torch().cuda.current_stream().cuda_stream)
+    t = _torch()
+    if t.cuda.is_initialized():  # the handle alone, without a Stream object
+        return ctypes.c_void_p(t._C._cuda_getCurrentRawStream(
+            t._C._cuda_getDevice()))
+    return ctypes.c_void_p(t.cuda.current_stream().cuda_stream)
 
 
 def volume_desc(t, volume_axes: Sequence[int] = (0, 1, 2)) -> kk_volume:

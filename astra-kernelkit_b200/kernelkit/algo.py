@@ -25,14 +25,36 @@ from .processing import preweight
 from .projector import BackProjector
 
 
-def _host_copy(dev):
-    """A host copy of a device tensor in pinned memory, as the reference
-    returns its results (``algo.py:46-48, 122-126``): the copy runs at
-    full bus speed and torch's host allocator reuses the pinned block."""
+def _host_copy(dev, host=None):
+    """A host copy of a device tensor in pinned memory (``host`` when
+    given), as the reference returns its results (``algo.py:46-48,
+    122-126``): the copy runs at full bus speed and torch's host allocator
+    reuses the pinned block."""
     t = _arrays.torch()
-    host = t.empty(dev.shape, dtype=dev.dtype, pin_memory=True)
+    if host is None:
+        host = t.empty(dev.shape, dtype=dev.dtype, pin_memory=True)
     host.copy_(dev)
     return host.numpy()
+
+
+def capture_graph(work):
+    """``work()`` recorded into a CUDA graph on a stream of its own (nothing
+    runs). Unlike ``torch.cuda.graph`` this does not empty torch's device
+    and pinned-host caches first, which every solve would then fill again
+    (pinning a result anew takes 5 to 10 ms)."""
+    t = _arrays.torch()
+    g = t.cuda.CUDAGraph()
+    s = t.cuda.Stream()
+    t.cuda.synchronize()
+    s.wait_stream(t.cuda.current_stream())
+    with t.cuda.stream(s):
+        g.capture_begin()
+        try:
+            work()
+        finally:
+            g.capture_end()
+    t.cuda.current_stream().wait_stream(s)
+    return g
 
 
 def _to_host(dev, out=None):
@@ -411,16 +433,8 @@ class SIRT:
 
     def capture(self):
         """Capture one iteration into a CUDA graph (no work runs)."""
-        t = _arrays.torch()
-        g = t.cuda.CUDAGraph()
-        s = t.cuda.Stream()
-        s.wait_stream(t.cuda.current_stream())
-        with t.cuda.stream(s):
-            with t.cuda.graph(g, stream=s):
-                self.step()
-        t.cuda.current_stream().wait_stream(s)
-        self._graph = g
-        return g
+        self._graph = capture_graph(self.step)
+        return self._graph
 
     def run(self, iters: int, use_graph: bool = True, callback=None,
             progress=None):
@@ -473,13 +487,17 @@ def sirt(projections: np.ndarray, projection_geometry: Any,
                 desc = "SIRT [" + "*" * (i % E) + "." * (E - i % E) + "]"
                 bar.set_description(f"{desc}: {state['norm']})")
             bar.update(1)
+    host = None
+    if not return_gpu:  # the result's block, pinned while the GPU works
+        host = _arrays.torch().empty(solver.x.shape, dtype=solver.x.dtype,
+                                     pin_memory=True)
     x = solver.run(iters, use_graph=use_graph, callback=callback,
                    progress=progress)
     if bar is not None:
         bar.close()
     if return_gpu:
         return x
-    return _host_copy(x)
+    return _host_copy(x, host)
 
 
 __all__ = ["fp", "bp", "fbp", "fdk", "sirt", "SIRT", "release_stream_buffers"]

@@ -28,7 +28,7 @@ from typing import Callable, Sequence
 import numpy as np
 
 from . import _arrays, _native
-from .algo import SIRT
+from .algo import SIRT, capture_graph
 
 
 class Autotuner:
@@ -234,15 +234,11 @@ class BatchedSIRT:
 
     def capture(self, iters: int = 1):
         """Capture ``iters`` iterations into one CUDA graph."""
-        t = self._t
-        g = t.cuda.CUDAGraph()
-        st = t.cuda.Stream()
-        st.wait_stream(t.cuda.current_stream())
-        with t.cuda.stream(st):
-            with t.cuda.graph(g, stream=st):
-                for _ in range(iters):
-                    self.step()
-        t.cuda.current_stream().wait_stream(st)
+        def work():
+            for _ in range(iters):
+                self.step()
+
+        g = capture_graph(work)
         self._graph = (g, iters)
         return g
 

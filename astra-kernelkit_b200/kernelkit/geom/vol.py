@@ -27,8 +27,10 @@ class VolumeGeometry:
         self.rotation = tuple(np.array(rotation, dtype=np.float32))
 
     def has_isotropic_voxels(self, atol: float = 1e-8) -> bool:
-        return bool(np.allclose(self.voxel_size, self.voxel_size[0],
-                                atol=atol))
+        size = self.voxel_size
+        if size[0] == size[1] == size[2]:
+            return True
+        return bool(np.allclose(size, size[0], atol=atol))
 
     def voxel_volume(self) -> float:
         """Volume of one voxel, from the extents (``geom/vol.py:79-89``)."""

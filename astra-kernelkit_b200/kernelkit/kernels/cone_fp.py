@@ -217,6 +217,16 @@ class RayDrivenConeFP(BaseKernel):
             return [x, y, z]
         return [[1.0, 1.0, v[0]]] * 3
 
+    def _output_scale_array(self, voxel_size) -> np.ndarray:
+        """``_output_scale`` as nine float32, kept for the last voxel size."""
+        key = tuple(voxel_size)
+        last = getattr(self, "_osc", None)
+        if last is None or last[0] != key:
+            last = (key, np.asarray(self._output_scale(voxel_size),
+                                    np.float32).reshape(9))
+            self._osc = last
+        return last[1]
+
     @staticmethod
     def geoms2params(projection_geometry, volume_geometry: VolumeGeometry
                      ) -> ConeFPParams:
@@ -406,8 +416,7 @@ class RayDrivenConeFP(BaseKernel):
             raise ValueError(
                 f"Projections of {pdesc.rows}x{pdesc.cols} pixels do not "
                 f"match the detector {int(det.rows[0])}x{int(det.cols[0])}.")
-        osc = np.asarray(self._output_scale(volume_geometry.voxel_size),
-                         np.float32).reshape(9)
+        osc = self._output_scale_array(volume_geometry.voxel_size)
         lay = self._volume_texture(vol, vdesc)
         self._launch(vdesc, pdesc, osc, lay, None, additive)
         del keep
@@ -519,8 +528,7 @@ class RayDrivenConeFP(BaseKernel):
         if work is None or work.numel() < need or work.device != vol.device:
             work = t.empty(need, dtype=t.float32, device=vol.device)
             self._adj_work = work
-        osc = np.asarray(self._output_scale(volume_geometry.voxel_size),
-                         np.float32).reshape(9)
+        osc = self._output_scale_array(volume_geometry.voxel_size)
         _native.check(_native.load().kk_cone_fp_adjoint(
             pdesc, vdesc, self._params_dev.data_ptr(), osc.ctypes.data,
             self._interp, self.slices_per_block, int(bool(additive)),
@@ -542,8 +550,7 @@ class RayDrivenConeFP(BaseKernel):
             if a.shape != out.shape or a.stride() != out.stride():
                 raise ValueError(f"`{name}` must have the layout of `out`.")
         res = _native.kk_fp_residual(measured.data_ptr(), weight.data_ptr())
-        osc = np.asarray(self._output_scale(volume_geometry.voxel_size),
-                         np.float32).reshape(9)
+        osc = self._output_scale_array(volume_geometry.voxel_size)
         lay = self._volume_texture(volume, vdesc)
         self._launch(vdesc, pdesc, osc, lay, res, False)
 

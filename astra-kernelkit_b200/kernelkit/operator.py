@@ -10,6 +10,8 @@ from abc import ABC, abstractmethod
 from typing import Any
 
 from . import _arrays
+from .kernels.cone_bp import VoxelDrivenConeBP
+from .kernels.cone_fp import RayDrivenConeFP
 from .projector import BackProjector, BaseProjector, ForwardProjector
 
 
@@ -35,9 +37,14 @@ class BaseOperator(ABC):
         raise NotImplementedError
 
 
-def _zeros(shape):
+def _output(shape, projector, additive):
+    """Output of an operator call: zeros, but uninitialised for this
+    package's own projectors when they overwrite every element."""
     t = _arrays.torch()
-    return t.zeros(shape, dtype=t.float32, device="cuda")
+    own = (type(projector) in (ForwardProjector, BackProjector)
+           and type(projector.kernel) in (RayDrivenConeFP, VoxelDrivenConeBP))
+    make = t.empty if own and not additive else t.zeros
+    return make(shape, dtype=t.float32, device="cuda")
 
 
 class ProjectorOperator(BaseOperator):
@@ -73,7 +80,7 @@ class ProjectorOperator(BaseOperator):
                 f"Input shape {tuple(input.shape)} does not match domain "
                 f"shape {self.domain_shape} of operator.")
         if out is None:
-            out = _zeros(self.range_shape)
+            out = _output(self.range_shape, self.projector, additive)
         self.projector.volume = input
         self.projector.projections = out
         self.projector(additive=additive)
@@ -108,7 +115,7 @@ class _Adjoint(BaseOperator):
                 f"Input shape {tuple(input.shape)} does not match domain "
                 f"shape {self.domain_shape} of operator.")
         if out is None:
-            out = _zeros(self.range_shape)
+            out = _output(self.range_shape, self.projector, additive)
         self.projector.projections = input
         self.projector.volume = out
         self.projector(additive)
@@ -166,7 +173,7 @@ class _ExactAdjoint(BaseOperator):
                 f"Input shape {tuple(input.shape)} does not match domain "
                 f"shape {self.domain_shape} of operator.")
         if out is None:
-            out = _zeros(self.range_shape)
+            out = _output(self.range_shape, self._op.projector, additive)
         fp = self._op.projector
         fp.kernel.transpose(input, fp._proj_geom_seq, fp.volume_geometry,
                             out, additive=additive)
