@@ -38,15 +38,18 @@ namespace kk {
 #define KK_FP_MINBLOCKS (48 / KK_FP_COLS)  // 40 registers
 #endif
 #ifndef KK_FP_PAD_MINBLOCKS
-#define KK_FP_PAD_MINBLOCKS (40 / KK_FP_COLS)  // the padded-copy kernel: 48 registers, no spills
+#define KK_FP_PAD_MINBLOCKS (36 / KK_FP_COLS)  // the padded-copy kernel: 56 registers
 #endif
 #ifndef KK_FP_PAIR_ROWS
-#define KK_FP_PAIR_ROWS 640  // most detector rows traced with column pairs (fp_blocks)
+#define KK_FP_PAIR_ROWS 1024  // most detector rows traced with column pairs (fp_blocks)
 #endif
 #ifndef KK_FP_GENERAL_MINBLOCKS
+// its instance for tilted detectors and column pairs: 192 x 192 x 160 x 300
+// tilted 3.10 ms, 3.26 with 64 registers
 #define KK_FP_GENERAL_MINBLOCKS (36 / KK_FP_COLS)
 #endif
 #ifndef KK_FP_EXACT_MINBLOCKS
+// exact weights, 48 registers: 192 x 192 x 180 x 250 3.30 ms, 3.55 with 56
 #define KK_FP_EXACT_MINBLOCKS (40 / KK_FP_COLS)
 #endif
 #ifndef KK_FP_PAD_TEX_UNROLL
@@ -134,14 +137,18 @@ __device__ __forceinline__ int span_class(float c0, float c1, int n) {
     return 1;
 }
 
+// Barrier of the FP_COLS tracing warps (the tile kernel's block has one more).
+__device__ __forceinline__ void fp_block_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * FP_COLS) : "memory");
+}
+
 template <typename TV, typename TP, bool TEX8, int EPI, int PATH, int RULE, bool AF = false, bool SUMS = false,
           bool PAD = false, bool GENERAL = false>
 __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, int rec, int a, int A, int D1, int D2,
-                                         int rule, bool a_fast, int r0, int c, int lane, bool cols2) {
+                                         int rule, bool a_fast, int r0, int c, int lane, bool cols2, float* tile) {
     // ray k of the thread: 32 rows further down, or FP_COLS columns on
     auto row = [&](int k) { return r0 + lane + (GENERAL && cols2 ? 0 : 32 * k); };
     auto col = [&](int k) { return c + (GENERAL && cols2 ? FP_COLS * k : 0); };
-    auto on_detector = [&](int k) { return row(k) < L.rows && (!GENERAL || col(k) < L.cols); };
     float src[3], cor[3], u[3], v[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -157,22 +164,47 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
     const float half1 = 0.5f * (float)n1, half2 = 0.5f * (float)n2;
     const float unit_inv = 1.f / weight_unit<TEX8>();
 
-    // output element of ray k
-    auto out_ptr = [&](int k) -> TP* {
-        const int64_t off = (int64_t)row(k) * L.ps[1] + (int64_t)col(k) * L.ps[2];
+    // The block's rays pass their sums through shared memory to threads that
+    // walk its FP_COLS (or twice as many) columns first, so that the warps'
+    // accesses to the projections, the residual's operands and the running
+    // sums cover runs of columns and not one element of 32 rows each. Those
+    // single elements took wavefronts of the L1 data stage, whose LSU and
+    // texture shares (35.5 and 57.1 %) bind the mixed launch: 512^3 x 720 x
+    // 768^2 152.2 -> 147.8 ms, 400 x 380 x 330 x 500 38.8 -> 37.2, 128 x 128
+    // x 100 x 180 0.605 -> 0.581; 56 registers instead of 48 (the epilogue's)
+    // then give 146.1 ms.
+    const int tid = threadIdx.x, width = GENERAL && cols2 ? 2 * FP_COLS : FP_COLS, ld_tile = width + 1;
+    const int c0 = c - (tid >> 5);
+    auto own = [&](int k) -> float& { return tile[(row(k) - r0) * ld_tile + col(k) - c0]; };
+    // visit(row, column, tile element) for this thread's share of the tile
+    auto visit = [&](auto visitor) {
+#pragma unroll
+        for (int i = 0; i < FP_RPT; ++i) {
+            const int e = tid + 32 * FP_COLS * i;
+            const int tr = GENERAL && cols2 ? e / (2 * FP_COLS) : e / FP_COLS;
+            const int tc = GENERAL && cols2 ? e % (2 * FP_COLS) : e % FP_COLS;
+            if (r0 + tr < L.rows && c0 + tc < L.cols) visitor(r0 + tr, c0 + tc, tile[tr * ld_tile + tc]);
+        }
+    };
+    auto out_ptr = [&](int r, int cc) -> TP* {
+        const int64_t off = (int64_t)r * L.ps[1] + (int64_t)cc * L.ps[2];
         return L.table ? (TP*)L.table[a] + off : (TP*)L.out + (int64_t)a * L.ps[0] + off;
     };
-    // running float32 sum of ray k between launches (16-bit outputs)
-    auto sum_ptr = [&](int k) -> float* {
-        return L.sums + ((int64_t)rec * L.rows + row(k)) * L.cols + col(k);
-    };
+    // running float32 sum between launches (16-bit outputs)
+    auto sum_ptr = [&](int r, int cc) -> float* { return L.sums + ((int64_t)rec * L.rows + r) * L.cols + cc; };
+    const bool resume = (SUMS && L.load_sums) || L.additive;
+    if (resume) {
+        visit([&](int r, int cc, float& v) { v = SUMS && L.load_sums ? *sum_ptr(r, cc) : ld_rw(out_ptr(r, cc)); });
+        fp_block_sync();
+    }
     RaySetup R[FP_RPT];
     float acc[FP_RPT];
 #pragma unroll
     for (int k = 0; k < FP_RPT; ++k) {
-        const bool valid = on_detector(k);
-        R[k] = ray_setup(src, cor, u, v, A, D1, D2, valid ? row(k) : 0, !GENERAL || valid ? col(k) : c, sc1, sc2);
-        acc[k] = !valid ? 0.f : (SUMS && L.load_sums) ? *sum_ptr(k) : L.additive ? ld_rw(out_ptr(k)) : 0.f;
+        // beyond the detector: a ray like its neighbours', whose sum nobody
+        // stores
+        R[k] = ray_setup(src, cor, u, v, A, D1, D2, min(row(k), L.rows - 1), min(col(k), L.cols - 1), sc1, sc2);
+        acc[k] = resume ? own(k) : 0.f;
     }
 
     const int s_end = min(nS, L.s_end);
@@ -461,19 +493,20 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
     }
 
 #pragma unroll
-    for (int k = 0; k < FP_RPT; ++k) {
-        if (!on_detector(k)) continue;
+    for (int k = 0; k < FP_RPT; ++k) own(k) = acc[k];
+    fp_block_sync();
+    visit([&](int r, int cc, float& v) {
         if (SUMS && L.store_sums) {
-            *sum_ptr(k) = acc[k];
-            continue;
+            *sum_ptr(r, cc) = v;
+            return;
         }
-        float out = acc[k];
+        float out = v;
         if (EPI == FP_RESIDUAL && L.final_pass) {
-            const int64_t e = (int64_t)a * L.ps[0] + (int64_t)row(k) * L.ps[1] + (int64_t)col(k) * L.ps[2];
+            const int64_t e = (int64_t)a * L.ps[0] + (int64_t)r * L.ps[1] + (int64_t)cc * L.ps[2];
             out = __fmul_rn(__fsub_rn(out, ld((const TP*)L.res_y + e)), ld((const TP*)L.res_w + e));
         }
-        st(out_ptr(k), out);
-    }
+        st(out_ptr(r, cc), out);
+    });
 }
 
 // PAD: the instance for a zero-padded volume copy (FpArgs.padded, offsets
@@ -492,7 +525,8 @@ __device__ __forceinline__ void fp_block(const FpArgs& L, int t) {
     const int rec = t % L.n_angles;
     const int rt = cols2 ? (L.rows - 1) / FP_ROWS_T : t / L.n_angles;
     const int c = ct * (cols2 ? 2 : 1) * FP_COLS + warp;
-    if (c >= L.cols) return;  // whole warp; the kernel has no block barrier
+    __shared__ float s_tile[FP_ROWS_T * (FP_COLS + 1)];
+    static_assert(FP_ROWS_T * (FP_COLS + 1) >= 32 * (2 * FP_COLS + 1), "tile of two columns per thread");
 
     const kk_fp_angle* P = L.angles + rec;
     const int a = __ldg(&P->index);  // projection written by this record
@@ -511,19 +545,19 @@ __device__ __forceinline__ void fp_block(const FpArgs& L, int t) {
     // layered texture is given, so both units share the work
     const bool use_tex = L.vtex && L.rank[A] == 2 && !(__ldg(&P->flags) & KK_FP_NO_TEXTURE);
     if (use_tex && a_fast)
-        fp_trace<TV, TP, TEX8, EPI, 3, 0, true, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
+        fp_trace<TV, TP, TEX8, EPI, 3, 0, true, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2, s_tile);
     else if (use_tex)
-        fp_trace<TV, TP, TEX8, EPI, 3, 0, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
+        fp_trace<TV, TP, TEX8, EPI, 3, 0, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2, s_tile);
     else if (TEX8 && shared && rule == 1)
-        fp_trace<TV, TP, TEX8, EPI, 2, 1, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
+        fp_trace<TV, TP, TEX8, EPI, 2, 1, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2, s_tile);
     else if (shared)
-        fp_trace<TV, TP, TEX8, EPI, 2, 0, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
+        fp_trace<TV, TP, TEX8, EPI, 2, 0, false, SUMS, PAD, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2, s_tile);
     else if (TEX8 && fast && rule == 1)
-        fp_trace<TV, TP, TEX8, EPI, 1, 1, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
+        fp_trace<TV, TP, TEX8, EPI, 1, 1, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2, s_tile);
     else if (fast)
-        fp_trace<TV, TP, TEX8, EPI, 1, 0, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
+        fp_trace<TV, TP, TEX8, EPI, 1, 0, false, SUMS, PAD && GENERAL, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2, s_tile);
     else
-        fp_trace<TV, TP, TEX8, EPI, 0, 0, false, SUMS, false, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2);
+        fp_trace<TV, TP, TEX8, EPI, 0, 0, false, SUMS, false, GENERAL>(L, P, rec, a, A, D1, D2, rule, a_fast, r0, c, lane, cols2, s_tile);
 }
 
 template <typename TV, typename TP, bool TEX8, int EPI, bool SUMS = false>
@@ -533,9 +567,9 @@ __global__ void __launch_bounds__(32 * FP_COLS, KK_FP_MINBLOCKS) cone_fp_kernel(
 
 // cone_fp_kernel on a zero-padded volume copy
 template <typename TV, typename TP, bool TEX8, int EPI, bool GENERAL>
-__global__ void __launch_bounds__(32 * FP_COLS, GENERAL ? KK_FP_GENERAL_MINBLOCKS
-                                                : TEX8  ? KK_FP_PAD_MINBLOCKS
-                                                        : KK_FP_EXACT_MINBLOCKS) cone_fp_pad_kernel(const FpArgs L) {
+__global__ void __launch_bounds__(32 * FP_COLS, !TEX8     ? KK_FP_EXACT_MINBLOCKS
+                                                : GENERAL ? KK_FP_GENERAL_MINBLOCKS
+                                                          : KK_FP_PAD_MINBLOCKS) cone_fp_pad_kernel(const FpArgs L) {
     fp_block<TV, TP, TEX8, EPI, false, true, GENERAL>(L, blockIdx.x);
 }
 
@@ -1042,8 +1076,9 @@ static bool launch_fp_sums(const FpArgs& base, bool tex8, cudaStream_t s, const 
 // instead, at the price of their D1 splits and registers (ms without and
 // with: 64^3 x 96 rows 0.162 / 0.157, 128 x 128 x 100 x 150 rows 0.704 /
 // 0.635, 192^3 x 288 rows 3.12 / 2.92, 277^3 x 416 rows 12.07 / 11.62, 362^3
-// x 544 rows 31.2 / 30.3). The idle share falls with the rows: beyond
-// KK_FP_PAIR_ROWS circular scans keep their kernel.
+// x 544 rows 31.2 / 30.3). The idle share falls with the rows (1/32 of the
+// rays at 1024) and the general kernel is 0.4 % slower on circular scans
+// (512^3 146.1 / 146.7 ms): beyond KK_FP_PAIR_ROWS they keep their kernel.
 static int64_t fp_blocks(FpArgs& L, bool pairs) {
     L.col_tiles = (L.cols + FP_COLS - 1) / FP_COLS;
     const int64_t row_tiles = (L.rows + FP_ROWS_T - 1) / FP_ROWS_T, per = (int64_t)L.n_angles * L.col_tiles;

@@ -95,8 +95,8 @@ def test_padded_pairs_options(kind, interp):
 
 @pytest.mark.parametrize("kind", ["circular", "tilted", "alldirs"])
 @pytest.mark.parametrize("rows,cols", [(1, 9), (32, 8), (33, 12), (64, 5),
-                                       (65, 4), (96, 13), (640, 7),
-                                       (641, 7)])
+                                       (65, 4), (96, 13), (961, 7),
+                                       (1025, 7)])
 def test_last_row_tiles(rows, cols, kind):
     vol = _volume((24, 26, 40))
     for interp in ("texture", "exact"):
