@@ -1153,11 +1153,11 @@ static int launch_fp(const FpArgs& L, int vdt, int pdt, bool tex8, cudaStream_t 
     // 16-bit storage (volume in bf16 or f16, projections in f16)
     KK_FP_CASE(KK_BF16, KK_F16, __nv_bfloat16, __half)
     KK_FP_CASE(KK_F16, KK_F16, __half, __half)
+    KK_FP_CASE(KK_F32, KK_F16, float, __half)
     if (EPI == FP_STORE) {
         KK_FP_CASE(KK_BF16, KK_F32, __nv_bfloat16, float)
         KK_FP_CASE(KK_F16, KK_F32, __half, float)
         KK_FP_CASE(KK_BF16, KK_BF16, __nv_bfloat16, __nv_bfloat16)
-        KK_FP_CASE(KK_F32, KK_F16, float, __half)
         KK_FP_CASE(KK_F32, KK_BF16, float, __nv_bfloat16)
     }
 #undef KK_FP_CASE
@@ -1169,18 +1169,20 @@ static int launch_fp(const FpArgs& L, int vdt, int pdt, bool tex8, cudaStream_t 
 // rank 0 fastest); src has the volume's own strides (per rank). Block =
 // blockDim.y padded rows (rank 1) of one padded plane (rank 2, block y);
 // threads stride along the padded rank-0 row, so both sides stream.
-template <typename T>
-__global__ void fp_pad_kernel(const T* __restrict__ src, T* __restrict__ dst, int n0, int n1, int n2, int64_t s0,
+// S to D: the same type (16-bit values are copied as they are) or a 16-bit
+// type to float.
+template <typename S, typename D>
+__global__ void fp_pad_kernel(const S* __restrict__ src, D* __restrict__ dst, int n0, int n1, int n2, int64_t s0,
                               int64_t s1, int64_t s2) {
     const int m0 = n0 + 4, m1 = n1 + 4;
     const int r = blockIdx.x * blockDim.y + threadIdx.y;
     if (r >= m1) return;
     const int i1 = r - 2, i2 = (int)blockIdx.y - 2;
-    T* row = dst + ((int64_t)blockIdx.y * m1 + r) * m0;
+    D* row = dst + ((int64_t)blockIdx.y * m1 + r) * m0;
     const bool row_in = (unsigned)i1 < (unsigned)n1 && (unsigned)i2 < (unsigned)n2;
     for (int p = threadIdx.x; p < m0; p += blockDim.x) {
         const int i0 = p - 2;
-        row[p] = row_in && (unsigned)i0 < (unsigned)n0 ? src[i0 * s0 + i1 * s1 + i2 * s2] : T(0);
+        row[p] = row_in && (unsigned)i0 < (unsigned)n0 ? (D)src[i0 * s0 + i1 * s1 + i2 * s2] : D(0);
     }
 }
 
@@ -1189,8 +1191,8 @@ __global__ void fp_pad_kernel(const T* __restrict__ src, T* __restrict__ dst, in
 // paired loops need every offset from the interior, within
 // [-interior, total - interior), in 32 bits: larger volumes keep tracing
 // the volume itself.
-static int fp_pad_volume(FpArgs& L, const kk_volume* vol, void* padded, int64_t padded_elems, cudaStream_t s,
-                         const char* who) {
+static int fp_pad_volume(FpArgs& L, const kk_volume* vol, void* padded, int64_t padded_elems, bool as_float,
+                         cudaStream_t s, const char* who) {
     int64_t n[3], st[3];
     for (int k = 0; k < 3; ++k) {
         n[L.rank[k]] = vol->shape[k];
@@ -1202,14 +1204,18 @@ static int fp_pad_volume(FpArgs& L, const kk_volume* vol, void* padded, int64_t 
         return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: the padded copy needs %lld elements", who, (long long)total);
     if (total >= ((int64_t)1 << 31) - 0x4B4000 - 2) return KK_OK;
     const dim3 block(128, 4), grid((unsigned)((n[1] + 4 + 3) / 4), (unsigned)(n[2] + 4));
-    const int es = vol->dtype == KK_F32 ? 4 : 2;
-    if (es == 4)
-        fp_pad_kernel<float><<<grid, block, 0, s>>>((const float*)vol->data, (float*)padded, (int)n[0],
-                                                   (int)n[1], (int)n[2], st[0], st[1], st[2]);
+    const int es = vol->dtype == KK_F32 || as_float ? 4 : 2;
+    auto copy = [&](auto src, auto dst) {
+        fp_pad_kernel<<<grid, block, 0, s>>>(src, dst, (int)n[0], (int)n[1], (int)n[2], st[0], st[1], st[2]);
+    };
+    if (vol->dtype == KK_F32)
+        copy((const float*)vol->data, (float*)padded);
+    else if (!as_float)
+        copy((const unsigned short*)vol->data, (unsigned short*)padded);
+    else if (vol->dtype == KK_BF16)
+        copy((const __nv_bfloat16*)vol->data, (float*)padded);
     else
-        fp_pad_kernel<unsigned short><<<grid, block, 0, s>>>((const unsigned short*)vol->data,
-                                                           (unsigned short*)padded, (int)n[0], (int)n[1],
-                                                           (int)n[2], st[0], st[1], st[2]);
+        copy((const __half*)vol->data, (float*)padded);
     const int64_t interior = 2 * (pst[0] + pst[1] + pst[2]);
     L.vol = (const char*)padded + interior * es;
     for (int k = 0; k < 3; ++k) L.vs[k] = pst[L.rank[k]];
@@ -1292,6 +1298,7 @@ extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, c
     int rc = fill_fp_args(L, vol, proj, angles, out_scale, opts->interp, opts->slab, who);
     if (rc) return rc;
     const bool tex8 = opts->interp == KK_INTERP_TEX8;
+    int vdt = vol->dtype;  // of the volume traced
     if (opts->vtex) {
         const kk_layered* vtex = opts->vtex;
         if (!tex8) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: a volume texture needs texture interpolation", who);
@@ -1308,8 +1315,10 @@ extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, c
         L.vtex = vtex->tex;
     }
     if (opts->padded && !(opts->flags & KK_FP_OPT_TILES)) {
-        rc = fp_pad_volume(L, vol, opts->padded, opts->padded_elems, (cudaStream_t)stream, who);
+        const bool as_float = (opts->flags & KK_FP_OPT_PADDED_FLOAT) != 0;
+        rc = fp_pad_volume(L, vol, opts->padded, opts->padded_elems, as_float, (cudaStream_t)stream, who);
         if (rc) return rc;
+        if (L.padded && as_float) vdt = KK_F32;
     }
     L.additive = opts->additive ? 1 : 0;
     if (opts->sums_elems < 0 || (opts->sums_elems > 0 && !opts->sums))
@@ -1324,9 +1333,9 @@ extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, c
         if (rc) return rc;
         L.res_y = res->y;
         L.res_w = res->weight;
-        return launch_fp<FP_RESIDUAL>(L, vol->dtype, proj->dtype, tex8, (cudaStream_t)stream, lo);
+        return launch_fp<FP_RESIDUAL>(L, vdt, proj->dtype, tex8, (cudaStream_t)stream, lo);
     }
-    return launch_fp<FP_STORE>(L, vol->dtype, proj->dtype, tex8, (cudaStream_t)stream, lo);
+    return launch_fp<FP_STORE>(L, vdt, proj->dtype, tex8, (cudaStream_t)stream, lo);
 }
 
 extern "C" int kk_fp_set_span(int32_t slices) {
@@ -1472,7 +1481,7 @@ extern "C" int kk_cone_fp_batched_ex(const kk_fp_problem* pr, int32_t n, int32_t
         pad = opts->padded[i] && (v[0] + 4) * (v[1] + 4) * (v[2] + 4) < ((int64_t)1 << 31) - 0x4B4000 - 2;
     }
     for (int i = 0; pad && i < n; ++i) {
-        const int rc = fp_pad_volume(args[i], &pr[i].vol, opts->padded[i], opts->padded_elems[i], st, who);
+        const int rc = fp_pad_volume(args[i], &pr[i].vol, opts->padded[i], opts->padded_elems[i], false, st, who);
         if (rc) return rc;
     }
     // launch p traces span p of every problem that has one; plain and

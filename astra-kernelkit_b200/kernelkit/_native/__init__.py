@@ -58,6 +58,8 @@ class kk_fp_options(ctypes.Structure):
 KK_FP_OPT_TILES = 1
 #: some records' detector rows do not share their in-slice coordinate
 KK_FP_OPT_GENERAL = 2
+#: the padded copy of a 16-bit volume is float32
+KK_FP_OPT_PADDED_FLOAT = 4
 
 
 class kk_bp_update(ctypes.Structure):

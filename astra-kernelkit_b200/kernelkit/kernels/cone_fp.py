@@ -436,6 +436,16 @@ class RayDrivenConeFP(BaseKernel):
             self._sums_buf = buf
         return buf.data_ptr(), buf.numel()
 
+    def _pads_float(self, vdesc) -> bool:
+        """Whether the padded copy of a 16-bit volume is float32: for
+        16-bit storage runs whose projections are traced in one launch (up
+        to 256 slices; longer rays pass their sums between launches through
+        a kernel that is faster on 2-byte texels). One conversion per texel
+        instead of one per sample: a bf16 projection at 256^3 x 360 x
+        384^2 10.9 -> 8.7 ms."""
+        return (self.half_texture and int(vdesc.dtype) != _native.KK_F32
+                and max(int(n) for n in vdesc.shape) <= 256)
+
     def _padded(self, vdesc):
         """(pointer, elements) of the zero-padded volume copy's buffer,
         allocated once per projector, device, volume shape and type."""
@@ -444,6 +454,8 @@ class RayDrivenConeFP(BaseKernel):
         t = _arrays.torch()
         dt = {_native.KK_F32: t.float32, _native.KK_BF16: t.bfloat16,
               _native.KK_F16: t.float16}[int(vdesc.dtype)]
+        if self._pads_float(vdesc):
+            dt = t.float32
         n = int(np.prod([int(x) + 4 for x in vdesc.shape]))
         if n >= 2 ** 31 - 0x4B4000 - 2:  # the kernels' 32-bit offsets
             return None, 0
@@ -472,7 +484,9 @@ class RayDrivenConeFP(BaseKernel):
         o.span = int(_DEFAULT_SPAN if self.slices_per_launch is None
                      else self.slices_per_launch)
         o.flags = ((_native.KK_FP_OPT_TILES if self.use_tiles else 0)
-                   | (_native.KK_FP_OPT_GENERAL if self._general else 0))
+                   | (_native.KK_FP_OPT_GENERAL if self._general else 0)
+                   | (_native.KK_FP_OPT_PADDED_FLOAT if vdesc is not None
+                      and self._pads_float(vdesc) else 0))
         o.vtex = None if lay is None else lay.handle
         o.residual = (None if residual is None
                       else ctypes.cast(ctypes.pointer(residual),

@@ -217,6 +217,10 @@ typedef struct {
  * those rays too (same results; the other kernel keeps more rays in flight
  * where every record shares). */
 #define KK_FP_OPT_GENERAL 2
+/* kk_fp_options.flags, with padded: the buffer holds float32 elements and
+ * the copy converts a 16-bit volume (same results: every sample converts
+ * its texels otherwise). */
+#define KK_FP_OPT_PADDED_FLOAT 4
 
 /* The forward projection with every option per call: kk_cone_fp,
  * kk_cone_fp_residual and kk_cone_fp_layered are this entry point with

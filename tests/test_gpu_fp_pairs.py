@@ -157,3 +157,34 @@ def test_batched_padded_copies():
     for o in (options(), options(skip=1)):
         for a, b in zip(run(o), ref):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["circular", "tilted"])
+@pytest.mark.parametrize("shape,floats", [((33, 47, 38), True),
+                                          ((257, 20, 18), False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_float_copies_of_16bit_volumes(dtype, shape, floats, kind):
+    """16-bit storage runs (half_texture): a float32 padded copy up to 256
+    slices, the volume's type beyond, and the unpadded projections bit for
+    bit, plain and with the residual epilogue."""
+    vol = _volume(shape, dtype)
+    vg = kk.resolve_volume_geometry(shape=shape, voxel_size=1.0)
+    pgs = _scan(kind, rows=44, cols=23)
+    y, w = (torch.rand((14, 44, 23), device="cuda").half() for _ in range(2))
+    outs = []
+    for padded in (True, False):
+        K = RayDrivenConeFP()
+        K.half_texture, K.padded_copy = True, padded
+        K.compile()
+        K.set_params(K.geoms2params(pgs, vg))
+        out = torch.zeros_like(y)
+        K(vol, pgs, vg, out, additive=False)
+        res = torch.zeros_like(y)
+        K.residual(vol, pgs, vg, res, y, w)
+        outs.append((out, res))
+        if padded:
+            want = torch.float32 if floats else dtype
+            assert K._pad_buf.dtype == want
+    assert float(outs[0][0].abs().sum()) > 0
+    assert torch.equal(outs[0][0], outs[1][0])
+    assert torch.equal(outs[0][1], outs[1][1])
