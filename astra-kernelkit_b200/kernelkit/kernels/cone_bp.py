@@ -47,11 +47,11 @@ class _StagePool:
     def add(self, kernel):
         with self.lock:
             self.users.add(kernel)
-        weakref.finalize(kernel, self._gone)
+        weakref.finalize(kernel, self._gone).atexit = False
 
     def _gone(self):
         with self.lock:
-            if not len(self.users):
+            if not list(self.users):  # len() still counts the one going
                 self.items.clear()
 
     def take(self, shape):

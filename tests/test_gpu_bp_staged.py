@@ -5,6 +5,7 @@ stages; two streams sharing one kernel; calls recorded into a CUDA graph,
 which keep the device-memory path."""
 from __future__ import annotations
 
+import gc
 import math
 
 import numpy as np
@@ -140,7 +141,12 @@ def test_textures_are_bounded_and_given_back():
     assert len(pool.items) == pool.LIMIT
     cone_bp.release_staging_textures()
     assert pool.items == []
+    keep.append(go(2, 35))
+    assert len(pool.items) == 1
     del keep
+    gc.collect()
+    if not list(pool.users):  # no kernel of another test is alive
+        assert pool.items == []
 
 
 def test_captured_calls_take_the_device_memory_path():
