@@ -976,16 +976,21 @@ using namespace kk;
 // span of slices of every ray's own slice axis (kk_fp_set_span sets
 // another span, or one launch). Each launch then reads a band of the
 // volume across the rays' slice axes, whose slab per row tile stays in L2
-// (at 512^3 / 720 angles / 768^2: DRAM reads down, FP 183.0 -> 168.4 ms
-// with two launches; 64-slice spans lose to the per-launch ray set-up).
+// (at 512^3 / 720 angles / 768^2: DRAM reads down; 64-slice spans lose to
+// the per-launch ray set-up).
 // The running float32 sums are carried in the projections between
 // launches: same operations and rounding as one launch. The automatic
-// span follows the longest axis, as measured with the padded-copy kernel:
-// one launch up to 256 slices (256^3 / 360 / 384^2: 9.7 ms, 10.4 ms with
-// 128 or 192), 192 up to 640 (512^3: 155.4 ms; 158.3 / 158.8 / 180.6 at
-// 128 / 256 / one launch), 128 beyond (1024^3 / 1440 / 1536^2: 2744 ms;
-// 2888 / 3059 / 3600 at 192 / 256 / one launch).
-static int fp_auto_span(int nmax) { return nmax <= 256 ? 256 : nmax <= 640 ? 192 : 128; }
+// span follows the longest axis: one launch up to 256 slices (256^3 x 360 x
+// 384^2: 8.95 ms, 9.39 with 128), equal spans of at most 208 slices up to 640
+// (512^3: three of 176 145.8 ms; spans of 192 146.7, 128 147.9, 256 157.2;
+// 400 x 380 x 330: two of 208 36.1 ms; spans of 192 37.2, 144 37.1, 128 38.3,
+// one launch 39.5), of at most 128 beyond (1024^3 x 1440 x 1536^2, before the
+// output tile: 2744 ms; 2888 / 3059 / 3600 at 192 / 256 / one launch).
+static int fp_auto_span(int nmax) {
+    const int most = nmax <= 256 ? 256 : nmax <= 640 ? 208 : 128;
+    const int launches = (nmax + most - 1) / most;
+    return (nmax + launches - 1) / launches;
+}
 // span of the legacy entry points (kk_fp_set_span), per calling thread:
 // 0 = automatic (fp_auto_span), < 0 = one launch, > 0 = slices
 static thread_local int g_fp_span = 0;

@@ -577,7 +577,7 @@ def set_slices_per_launch(slices: int = 0) -> None:
     """How many slices of every ray's own slice axis one forward-projection
     launch traces (float32 projections) for projectors that do not set
     ``slices_per_launch`` themselves: 0 = the library's automatic span
-    (one launch up to 256 slices, 192 slices up to 640, 128 beyond), -1 =
+    (one launch up to 256 slices, equal spans of at most 208 up to 640, 128 beyond), -1 =
     the whole ray in one launch. Results are the same bit for bit;
     shorter spans keep the volume band each launch reads in L2."""
     global _DEFAULT_SPAN

@@ -171,9 +171,9 @@ typedef struct {
                            in the projections, so the result is bit for bit
                            that of one launch) and each launch reads a band
                            of the volume that stays in L2. 0: by the
-                           longest axis (one launch up to 256 slices, 192-
-                           slice spans up to 640, 128 beyond), -1: one
-                           launch */
+                           longest axis (one launch up to 256 slices,
+                           equal spans of at most 208 up to 640, of at most
+                           128 beyond), -1: one launch */
     int32_t flags;      /* KK_FP_OPT_* bits */
     const kk_layered* vtex;          /* NULL, or a layered copy of the
                                         volume as for kk_cone_fp_layered */
