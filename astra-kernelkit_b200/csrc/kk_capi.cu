@@ -12,11 +12,16 @@
 
 static thread_local char g_last_error[512] = "";
 
+// The status and message of a failed call. A CUDA error is reported once, by
+// the call that met it: the runtime keeps it as its last error too, which
+// kk_check_launch() of a later call would otherwise take for that call's own
+// (a caller may go on after a failed allocation).
 int kk_fail(int status, const char* fmt, ...) {
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(g_last_error, sizeof(g_last_error), fmt, ap);
     va_end(ap);
+    if (status == KK_ERR_CUDA) cudaGetLastError();
     return status;
 }
 
