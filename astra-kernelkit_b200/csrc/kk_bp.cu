@@ -30,23 +30,36 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
-// bilinear<false>() from a layer of the texture: the four texels of the
-// footprint come from one texture gather at its centre (texels beyond the
-// border read zero), so the lanes of a warp, whose rows differ, do not each
-// fetch their own lines (128 x 128 x 100 x 180 x 150 x 192: 2.34 -> 0.98 ms
-// with the copy into the texture, 0.43 ms for the texture's own weights; the
-// weights' arithmetic now takes the issue slots). floor() by rounding down at 2^23: same result, without the
+// bilinear<false>() from a tile of a kk_gather array whose texel (0, 0) is at
+// org - 1: the four texels of the footprint come from one texture gather at
+// its centre, so the lanes of a warp, whose rows differ, do not each fetch
+// their own lines (128 x 128 x 100 x 180 x 150 x 192: 2.34 -> 0.98 ms with
+// the copy into the texture, 0.43 ms for the texture's own weights; the
+// weights' arithmetic now takes the issue slots). Coordinates beyond the
+// tile's two zero rows and columns move onto them, where the sample is zero
+// as well. floor() by rounding down at 2^23: same result, without the
 // conversion unit.
-__device__ __forceinline__ float gather_exact(cudaTextureObject_t tex, float V, float U, int layer) {
-    const float vb = fminf(fmaxf(V, -COORD_LIMIT), COORD_LIMIT) - 0.5f;
-    const float ub = fminf(fmaxf(U, -COORD_LIMIT), COORD_LIMIT) - 0.5f;
+__device__ __forceinline__ float gather_exact(cudaTextureObject_t tex, float V, float U, float rows, float cols,
+                                              float2 org) {
+    const float vb = fminf(fmaxf(V, -1.f), rows + 1.f) - 0.5f;
+    const float ub = fminf(fmaxf(U, -1.f), cols + 1.f) - 0.5f;
     const float fv = __fadd_rd(vb, 12582912.f) - 12582912.f, fu = __fadd_rd(ub, 12582912.f) - 12582912.f;
     const float wa = vb - fv, wb = ub - fu;
-    float t10, t11, t01, t00;  // [row][column], counter-clockwise from the lower left
-    asm("tld4.r.a2d.v4.f32.f32 {%0, %1, %2, %3}, [%4, {%5, %6, %7, %7}];"
-        : "=f"(t10), "=f"(t11), "=f"(t01), "=f"(t00)
-        : "l"(tex), "r"(layer), "f"(fu + 1.f), "f"(fv + 1.f));
-    return combine4<false>(t00, t01, t10, t11, weights4<false>(wa, wb, 0, true));
+    // counter-clockwise from the lower left: [row][column] 10, 11, 01, 00
+    const float4 t = tex2Dgather<float4>(tex, fu + org.x, fv + org.y, 0);
+    return combine4<false>(t.w, t.z, t.x, t.y, weights4<false>(wa, wb, 0, true));
+}
+
+// The same from a layer of a layered array, whose texels CUDA lets kernels
+// read one by one only (half the rate of the gather: 256^3 x 360 x 384^2
+// 20.2 and 10.3 ms, from device memory 39.8).
+__device__ __forceinline__ float surface_exact(cudaSurfaceObject_t surf, float V, float U, int layer) {
+    const Split a = split_coord<false>(V), b = split_coord<false>(U);
+    const int x = b.i * (int)sizeof(float);
+    auto texel = [&](int dr, int dc) {
+        return surf2DLayeredread<float>(surf, x + dc * (int)sizeof(float), a.i + dr, layer, cudaBoundaryModeZero);
+    };
+    return combine4<false>(texel(0, 0), texel(0, 1), texel(1, 0), texel(1, 1), weights4<false>(a.w, b.w, 0, true));
 }
 
 // Angles of a chunk that cannot reach the block's voxels: thread tid tests
@@ -129,6 +142,7 @@ __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz
     constexpr int LAYERS = SPLIT ? KK_BP_CHUNKS_PER_LAUNCH : 1, THREADS = BP_TILE_2 * TY;
     __shared__ kk_bp_angle s_angles[LAYERS][BP_CHUNK];
     __shared__ unsigned char s_missed[LAYERS][BP_CHUNK / 4];  // four angles of bp_block_misses each
+    __shared__ float2 s_org[FETCH == FETCH_GATHER ? BP_CHUNK : 1];  // one past texel (0, 0) of each angle's tile
     const int layer = SPLIT ? threadIdx.z : 0;
     kk_bp_angle* sp = s_angles[layer];
     unsigned char* s_miss = s_missed[layer];
@@ -180,6 +194,10 @@ __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz
         __syncthreads();
         for (int k = tid; k < nj * 12; k += THREADS)
             ((float*)sp)[k] = __ldg((const float*)(L.angles + j0) + k);
+        if (FETCH == FETCH_GATHER && tid < nj) {
+            const int j = j0 + tid;
+            s_org[tid] = make_float2((float)(j % L.tiles_x * (L.cols + 2) + 3), (float)(j / L.tiles_x * (L.rows + 2) + 3));
+        }
 #pragma unroll
         for (int q = 0; q < BP_CHUNK; q += THREADS / 8) {
             const unsigned miss = bp_block_misses<TY>(L, j0 + q, nj - q, bx, by, g0, cnt, tid);
@@ -204,7 +222,9 @@ __device__ __forceinline__ void bp_block(const BpArgs& L, int bx, int by, int bz
             float dn = fmaf(Z, q.den[2], fmaf(Y, q.den[1], fmaf(X, q.den[0], q.den[3])));
             const float du = q.num_u[m0], dv = q.num_v[m0], dd = q.den[m0];
             auto sample = [&](float u, float v) {
-                return FETCH == FETCH_TEX ? tex2DLayered<float>(L.tex, u, v, j) : gather_exact(L.tex, v, u, j);
+                return FETCH == FETCH_TEX    ? tex2DLayered<float>(L.tex, u, v, j)
+                       : FETCH == FETCH_SURF ? surface_exact((cudaSurfaceObject_t)L.tex, v, u, j)
+                                             : gather_exact(L.tex, v, u, (float)L.rows, (float)L.cols, s_org[jj]);
             };
             if (FETCH != FETCH_GLOBAL && cnt == BP_GROUP) {
                 // full groups: two voxels at a time, their accumulation in
@@ -343,6 +363,21 @@ __global__ void layered_fill_kernel(const float* src, const uint64_t* table, int
     const float* p = (table ? (const float*)table[a] : src + (int64_t)a * sa) + (int64_t)c * sc;
     for (int r = blockIdx.y * 8; r < min(rows, (int)blockIdx.y * 8 + 8); ++r)
         surf2DLayeredwrite(__ldg(p + (int64_t)r * sr), surf, c * (int)sizeof(float), r, layer);
+}
+
+// The same into the tiles of a kk_gather array, with the two zero rows and
+// columns around each. Tiles share them: neighbours write the same zeros.
+__global__ void gather_fill_kernel(const float* src, const uint64_t* table, int64_t sa, int64_t sr, int64_t sc,
+                                   int rows, int cols, int first, int tiles_x, cudaSurfaceObject_t surf) {
+    const int c = (int)(blockIdx.x * 128 + threadIdx.x) - 2, layer = blockIdx.z, a = first + layer;
+    if (c >= cols + 2) return;
+    const float* p = (table ? (const float*)table[a] : src + (int64_t)a * sa) + (int64_t)c * sc;
+    const int x = (layer % tiles_x * (cols + 2) + 2 + c) * (int)sizeof(float), y = layer / tiles_x * (rows + 2) + 2;
+    const int r0 = (int)blockIdx.y * 8 - 2;
+    for (int r = r0; r < min(rows + 2, r0 + 8); ++r) {
+        const bool in = (unsigned)r < (unsigned)rows && (unsigned)c < (unsigned)cols;
+        surf2Dwrite(in ? __ldg(p + (int64_t)r * sr) : 0.f, surf, x, y + r);
+    }
 }
 
 // cone_bp_kernel through the texture with a layer of threads per 32-angle
@@ -775,6 +810,115 @@ extern "C" int kk_layered_fill(kk_layered* t, const kk_projections* src, int64_t
     return kk_check_launch(who);
 }
 
+// ---------------------------------------------------------------------------
+// projections for texture gathers
+// ---------------------------------------------------------------------------
+
+extern "C" int kk_gather_create(int64_t layers, int64_t height, int64_t width, kk_gather** out) {
+    const char* who = "kk_gather_create";
+    if (!out) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: out is NULL", who);
+    *out = nullptr;
+    if (layers <= 0 || height <= 0 || width <= 0 || layers > 2048 || height >= (int64_t)COORD_LIMIT ||
+        width >= (int64_t)COORD_LIMIT)
+        return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: bad extent (%lld, %lld, %lld)", who, (long long)layers,
+                       (long long)height, (long long)width);
+    int dev = 0, most_x = 0, most_y = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most_x, cudaDevAttrMaxTexture2DGatherWidth, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most_y, cudaDevAttrMaxTexture2DGatherHeight, dev);
+    if (e != cudaSuccess) return kk_fail(KK_ERR_CUDA, "%s: %s", who, cudaGetErrorString(e));
+    // as many tiles on top of each other as fit, evened out over the columns
+    int64_t ny = std::min<int64_t>(layers, (most_y - 2) / (height + 2));
+    const int64_t nx = ny > 0 ? (layers + ny - 1) / ny : 0;
+    if (ny < 1 || nx * (width + 2) + 2 > most_x)
+        return kk_fail(KK_ERR_UNSUPPORTED, "%s: %lld tiles of %lld x %lld do not fit an array of %d x %d", who,
+                       (long long)layers, (long long)height, (long long)width, most_y, most_x);
+    ny = (layers + nx - 1) / nx;
+    const cudaChannelFormatDesc ch = cudaCreateChannelDesc<float>();
+    kk_gather* t = new kk_gather();
+    t->tex = 0;
+    t->surf = 0;
+    t->layers = layers;
+    t->height = height;
+    t->width = width;
+    t->tiles_x = (int)nx;
+    e = cudaMallocArray(&t->array, &ch, (size_t)(nx * (width + 2) + 2), (size_t)(ny * (height + 2) + 2),
+                        cudaArrayTextureGather | cudaArraySurfaceLoadStore);
+    if (e != cudaSuccess) {
+        delete t;
+        return kk_fail(KK_ERR_CUDA, "%s: %s", who, cudaGetErrorString(e));
+    }
+    cudaResourceDesc rd = {};
+    rd.resType = cudaResourceTypeArray;
+    rd.res.array.array = t->array;
+    cudaTextureDesc td = {};
+    td.addressMode[0] = td.addressMode[1] = cudaAddressModeBorder;
+    td.filterMode = cudaFilterModeLinear;
+    td.readMode = cudaReadModeElementType;
+    e = cudaCreateTextureObject(&t->tex, &rd, &td, nullptr);
+    if (e == cudaSuccess) e = cudaCreateSurfaceObject(&t->surf, &rd);
+    if (e != cudaSuccess) {
+        kk_gather_destroy(t);
+        return kk_fail(KK_ERR_CUDA, "%s: %s", who, cudaGetErrorString(e));
+    }
+    *out = t;
+    return KK_OK;
+}
+
+extern "C" int kk_gather_destroy(kk_gather* t) {
+    if (!t) return KK_OK;
+    if (t->surf) cudaDestroySurfaceObject(t->surf);
+    if (t->tex) cudaDestroyTextureObject(t->tex);
+    cudaFreeArray(t->array);
+    delete t;
+    return KK_OK;
+}
+
+extern "C" int kk_gather_fill(kk_gather* t, const kk_projections* src, int64_t first, int64_t count, void* stream) {
+    const char* who = "kk_gather_fill";
+    if (!t) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: texture is NULL", who);
+    int rc = check_projections(src, who);
+    if (rc) return rc;
+    if (src->dtype != KK_F32) return kk_fail(KK_ERR_UNSUPPORTED, "%s: float32 projections only", who);
+    if (src->rows != t->height || src->cols != t->width || first < 0 || count < 1 || count > t->layers ||
+        first + count > src->n_angles)
+        return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: projections [%lld, %lld) do not fit the texture", who,
+                       (long long)first, (long long)(first + count));
+    const dim3 grid((unsigned)((src->cols + 4 + 127) / 128), (unsigned)((src->rows + 4 + 7) / 8), (unsigned)count);
+    gather_fill_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>((const float*)src->data, src->table, src->stride[0],
+                                                               src->stride[1], src->stride[2], (int)src->rows,
+                                                               (int)src->cols, (int)first, t->tiles_x, t->surf);
+    return kk_check_launch(who);
+}
+
+extern "C" int kk_cone_bp_gather(const kk_gather* t, int64_t n_angles, const kk_volume* vol, const kk_bp_angle* angles,
+                                 float out_scale, int32_t additive, void* stream) {
+    const char* who = "kk_cone_bp_gather";
+    if (!t) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: texture is NULL", who);
+    if (n_angles < 1 || n_angles > t->layers)
+        return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: %lld angles of %lld layers", who, (long long)n_angles,
+                       (long long)t->layers);
+    kk_projections p = {};
+    p.data = (void*)1;  // texels come from the texture; the descriptor carries the extent
+    p.n_angles = n_angles;
+    p.rows = t->height;
+    p.cols = t->width;
+    p.stride[0] = p.stride[1] = p.stride[2] = 1;
+    p.dtype = KK_F32;
+    BpArgs L;
+    const int rc = fill_bp_args(L, &p, vol, angles, out_scale, KK_INTERP_EXACT, who);
+    if (rc) return rc;
+    if (vol->dtype != KK_F32) return kk_fail(KK_ERR_UNSUPPORTED, "%s: float32 volume only", who);
+    L.proj = nullptr;
+    L.tex = t->tex;
+    L.tiles_x = t->tiles_x;
+    bp_chunks(L, true, additive != 0, false, [&](const BpArgs& c) {
+        cone_bp_kernel<float, float, false, BP_STORE, FETCH_GATHER>
+            <<<bp_grid(c), dim3(BP_TILE_2, BP_TILE_1), 0, (cudaStream_t)stream>>>(c);
+    });
+    return kk_check_launch(who);
+}
+
 static int layered_args(BpArgs& L, const kk_layered* t, const kk_volume* vol, const kk_bp_angle* angles,
                         float out_scale, const char* who) {
     if (!t) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: texture is NULL", who);
@@ -810,12 +954,13 @@ extern "C" int kk_cone_bp_layered_ex(const kk_layered* t, int64_t n_angles, cons
     if (interp == KK_INTERP_EXACT && (vdt != KK_F32 || t->dtype != KK_F32))
         return kk_fail(KK_ERR_UNSUPPORTED, "%s: exact weights take a float32 texture and volume", who);
     if (n_angles > 0) L.n_angles = (int)n_angles;
+    if (interp == KK_INTERP_EXACT) L.tex = (cudaTextureObject_t)t->surf;
     L.work = work;
     const dim3 block(BP_TILE_2, BP_TILE_1);
     const cudaStream_t s = (cudaStream_t)stream;
     bp_chunks(L, vdt == KK_F32, additive != 0, false, [&](const BpArgs& c) {
         if (interp == KK_INTERP_EXACT)
-            cone_bp_kernel<float, float, false, BP_STORE, FETCH_GATHER><<<bp_grid(c), block, 0, s>>>(c);
+            cone_bp_kernel<float, float, false, BP_STORE, FETCH_SURF><<<bp_grid(c), block, 0, s>>>(c);
         else if (vdt == KK_F32)
             launch_bp_tex<float, BP_STORE>(c, s);
         else if (vdt == KK_BF16)

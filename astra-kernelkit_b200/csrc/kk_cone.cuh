@@ -87,7 +87,8 @@ struct BpArgs {
     const void* upd_mask;
     float vmin, vmax;
     int has_min, has_max;
-    cudaTextureObject_t tex;  // layered texture of the projections (FETCH_TEX)
+    cudaTextureObject_t tex;  // texture of the projections (FETCH_SURF: the surface)
+    int tiles_x;              // FETCH_GATHER: tiles per row of the array
     int j_begin, j_end;       // angles of this launch (one accumulation chunk)
     int load_mode;            // running sum starts from 0 (LOAD_ZERO), vol, work
     int store_mode;           // partial sum goes to vol (STORE_VOL) or work
@@ -101,8 +102,9 @@ enum BpLoad { LOAD_ZERO = 0, LOAD_VOL = 1, LOAD_WORK = 2 };
 enum BpStore { STORE_VOL = 0, STORE_WORK = 1, STORE_FINAL = 2 };
 
 // texels from device memory, through the texture's own filter, or the four
-// texels of the footprint from the texture with exact weights
-enum BpFetch { FETCH_GLOBAL = 0, FETCH_TEX = 1, FETCH_GATHER = 2 };
+// texels of the footprint with exact weights: by one texture gather from a
+// 2D array of tiles, or by four surface reads from a layered array
+enum BpFetch { FETCH_GLOBAL = 0, FETCH_TEX = 1, FETCH_GATHER = 2, FETCH_SURF = 3 };
 
 }  // namespace kk
 
@@ -113,6 +115,18 @@ struct kk_layered {
     cudaSurfaceObject_t surf;  // float32 arrays: writable by kernels (FDK filter)
     int64_t layers, height, width;
     int32_t dtype;
+};
+
+// 2D CUDA array for texture gathers, which CUDA has for arrays of two
+// dimensions only: the layers are tiles of (height + 2) x (width + 2) texels,
+// tiles_x to a row, whose first two rows and columns are zero, as are two
+// more rows and columns after the last tiles
+struct kk_gather {
+    cudaArray_t array;
+    cudaTextureObject_t tex;
+    cudaSurfaceObject_t surf;
+    int64_t layers, height, width;
+    int tiles_x;
 };
 
 namespace kk {

@@ -123,7 +123,8 @@ EXPORTS = ("kk_cone_fp_ex", "kk_fp_launches_ex", "kk_wait_timeouts",
            "kk_cone_bp", "kk_cone_bp_static",
            "kk_cone_bp_update", "kk_layered_create", "kk_layered_copy",
            "kk_layered_destroy", "kk_layered_fill", "kk_cone_bp_layered",
-           "kk_cone_bp_layered_ex",
+           "kk_cone_bp_layered_ex", "kk_gather_create", "kk_gather_destroy",
+           "kk_gather_fill", "kk_cone_bp_gather",
            "kk_cone_bp_layered_update", "kk_preweight", "kk_filter_rows",
            "kk_reciprocal", "kk_sirt_update", "kk_fp_set_span",
            "kk_fp_launches", "kk_last_error",
@@ -182,6 +183,10 @@ def load():
     L.kk_layered_fill.argtypes = [vp, P(kk_projections), i64, i64, vp]
     L.kk_cone_bp_layered_ex.argtypes = [vp, i64, P(kk_volume), vp, f32, i32,
                                         i32, vp, vp]
+    L.kk_gather_create.argtypes = [i64, i64, i64, P(vp)]
+    L.kk_gather_destroy.argtypes = [vp]
+    L.kk_gather_fill.argtypes = [vp, P(kk_projections), i64, i64, vp]
+    L.kk_cone_bp_gather.argtypes = [vp, i64, P(kk_volume), vp, f32, i32, vp]
     L.kk_cone_bp_layered.argtypes = [vp, P(kk_volume), vp, f32, i32, vp, vp]
     L.kk_cone_bp_layered_update.argtypes = [vp, P(kk_volume), vp, f32,
                                             P(kk_bp_update), vp, vp]
@@ -338,4 +343,21 @@ class Layered:
         h = getattr(self, "handle", None)
         if h is not None and h.value and _lib is not None:
             _lib.kk_layered_destroy(h)
+            self.handle = None
+
+
+class Gather:
+    """Owner of a ``kk_gather`` array of projections (destroyed with the
+    object)."""
+
+    def __init__(self, layers, height, width):
+        self.shape = (int(layers), int(height), int(width))
+        h = ctypes.c_void_p()
+        check(load().kk_gather_create(*self.shape, ctypes.byref(h)))
+        self.handle = h
+
+    def __del__(self):
+        h = getattr(self, "handle", None)
+        if h is not None and h.value and _lib is not None:
+            _lib.kk_gather_destroy(h)
             self.handle = None

@@ -54,13 +54,15 @@ class _StagePool:
             if not list(self.users):  # len() still counts the one going
                 self.items.clear()
 
-    def take(self, shape):
-        """A texture of at least ``shape[0]`` layers, with the current
-        stream made to wait for its last use, or None without memory for
-        one. The caller holds the lock."""
+    def take(self, shape, gather=False):
+        """A texture (``gather``: one for exact weights) of at least
+        ``shape[0]`` layers, with the current stream made to wait for its
+        last use, or None without memory for one. The caller holds the
+        lock."""
         t = _arrays.torch()
         stream = t.cuda.current_stream()
         fit = [i for i in self.items if i["device"] == stream.device
+               and isinstance(i["texture"], _native.Gather) == gather
                and i["texture"].shape[1:] == shape[1:]
                and i["texture"].shape[0] >= shape[0]]
         ready = [i for i in fit if i["stream"] == stream or i["used"].query()]
@@ -73,7 +75,8 @@ class _StagePool:
                 old = next((i for i in self.items if i not in fit), None)
                 self.items.remove(old or self.items[0])
             try:
-                tex = _native.Layered(*shape, _native.KK_F32)
+                tex = (_native.Gather(*shape) if gather else
+                       _native.Layered(*shape, _native.KK_F32))
             except (_native.KernelKitError, ValueError):
                 return None
             item = {"texture": tex, "device": stream.device,
@@ -266,19 +269,30 @@ class VoxelDrivenConeBP(BaseKernel):
         L = _native.load()
         n = int(pdesc.n_angles)
         shape = (min(_STAGE_ANGLES, n), int(pdesc.rows), int(pdesc.cols))
+        gather = self._interp == _native.KK_INTERP_EXACT
         with _STAGES.lock:
-            item = _STAGES.take(shape)
+            try:
+                item = _STAGES.take(shape, gather)
+            except NotImplementedError:  # frames too large for gathers
+                gather = False
+                item = _STAGES.take(shape)
             if item is None:
                 return False
             tex = item["texture"].handle
             stream = _native.current_stream()
             for a in range(0, n, _STAGE_ANGLES):
                 m = min(_STAGE_ANGLES, n - a)
+                params = self._params_dev.data_ptr() + a * 12 * 4
+                add = int(bool(additive) or a > 0)
+                if gather:
+                    _native.check(L.kk_gather_fill(tex, pdesc, a, m, stream))
+                    _native.check(L.kk_cone_bp_gather(
+                        tex, m, vdesc, params, float(vox_vol), add, stream))
+                    continue
                 _native.check(L.kk_layered_fill(tex, pdesc, a, m, stream))
                 _native.check(L.kk_cone_bp_layered_ex(
-                    tex, m, vdesc, self._params_dev.data_ptr() + a * 12 * 4,
-                    float(vox_vol), self._interp,
-                    int(bool(additive) or a > 0), 0, stream))
+                    tex, m, vdesc, params, float(vox_vol), self._interp, add,
+                    0, stream))
             item["used"].record()
         return True
 

@@ -344,12 +344,28 @@ KK_API int kk_layered_fill(kk_layered* tex, const kk_projections* src,
 
 /* kk_cone_bp_layered on the first n_angles layers (0: all), with the
  * texture's own interpolation (KK_INTERP_TEX8) or exact weights on its
- * texels (KK_INTERP_EXACT; float32 texture and volume). */
+ * texels (KK_INTERP_EXACT; float32 texture and volume; kk_cone_bp_gather
+ * reads them twice as fast). */
 KK_API int kk_cone_bp_layered_ex(const kk_layered* tex, int64_t n_angles,
                                  const kk_volume* vol,
                                  const kk_bp_angle* angles, float out_scale,
                                  int32_t interp, int32_t additive,
                                  float* work, void* stream);
+
+/* Projections for backprojection with exact weights by texture gathers: one
+ * float32 tile per angle in a 2D CUDA array (gathers are defined for arrays
+ * of two dimensions only). KK_ERR_UNSUPPORTED when the device's gather
+ * limits (32768 x 32768) do not hold `layers` tiles. kk_gather_fill and
+ * kk_cone_bp_gather are kk_layered_fill and kk_cone_bp_layered_ex on it. */
+typedef struct kk_gather kk_gather;
+KK_API int kk_gather_create(int64_t layers, int64_t height, int64_t width,
+                            kk_gather** out);
+KK_API int kk_gather_destroy(kk_gather* tex);
+KK_API int kk_gather_fill(kk_gather* tex, const kk_projections* src,
+                          int64_t first, int64_t count, void* stream);
+KK_API int kk_cone_bp_gather(const kk_gather* tex, int64_t n_angles,
+                             const kk_volume* vol, const kk_bp_angle* angles,
+                             float out_scale, int32_t additive, void* stream);
 
 /* kk_cone_bp / kk_cone_bp_update sampling the layered texture. */
 KK_API int kk_cone_bp_layered(const kk_layered* tex, const kk_volume* vol,

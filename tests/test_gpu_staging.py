@@ -1,5 +1,5 @@
-"""Staging textures of the backprojection when something else goes on: no
-memory for a texture."""
+"""Staging textures of the backprojection: the tiles that exact weights
+gather from, no memory for a texture."""
 from __future__ import annotations
 
 import math
@@ -69,10 +69,60 @@ def test_no_memory_for_a_texture(interp, monkeypatch):
 
     class Native:
         def __getattr__(self, name):
-            return _NoMemory if name == "Layered" else getattr(_native, name)
+            return (_NoMemory if name in ("Layered", "Gather")
+                    else getattr(_native, name))
 
     monkeypatch.setattr(cone_bp, "_native", Native())
     out = torch.empty(SHAPE, device="cuda")
     K([f.clone() for f in y], out, vg, additive=False)
     assert cone_bp._STAGES.items == []
     assert torch.equal(out, _direct(K, y, vg))
+
+
+def _same(a, b):
+    nan = torch.isnan(a)
+    return (torch.equal(nan, torch.isnan(b))
+            and torch.equal(a[~nan], b[~nan]))
+
+
+@pytest.mark.parametrize("n,rows,cols", [
+    (1, 1, 1), (33, 2, 45), (131, 400, 23),  # 2 tiles to a row of the array
+    (40, 41, 1500), (97, 700, 301)])
+def test_gather_tiles(n, rows, cols):
+    """The same operations on the same texels as from device memory, bit for
+    bit; frames of infinities, NaNs and the largest values next to each
+    other stay where they are."""
+    K, vg, y = _case(n, "exact", rows, cols)
+    y[1::5], y[2::7], y[3::11] = math.inf, math.nan, 3e38
+    y[0, 0], y[0, -1], y[0, :, 0], y[0, :, -1] = 1.0, 2.0, 3.0, 4.0
+    K._stages = lambda *a: True  # also where the copy does not pay
+    out = torch.empty(SHAPE, device="cuda")
+    cone_bp.release_staging_textures()
+    K(y, out, vg, additive=False)
+    assert [type(i["texture"]) for i in cone_bp._STAGES.items] == [
+        _native.Gather]
+    assert _same(out, _direct(K, y, vg))
+
+
+@pytest.mark.parametrize("n", [20, 131])
+def test_frames_too_large_for_gathers(n, monkeypatch):
+    """Staged in a layered texture, whose texels are read one by one."""
+    with pytest.raises(NotImplementedError):
+        _native.Gather(1000, 16000, 16000)
+    K, vg, y = _case(n, "exact")
+    y[1::5], y[0, 0], y[0, :, -1] = math.inf, 1.0, 4.0
+
+    class Native:
+        class Gather:
+            def __init__(self, *shape):
+                raise NotImplementedError
+
+        def __getattr__(self, name):
+            return getattr(_native, name)
+
+    cone_bp.release_staging_textures()
+    monkeypatch.setattr(cone_bp, "_native", Native())
+    out = torch.empty(SHAPE, device="cuda")
+    K(y, out, vg, additive=False)
+    assert len(cone_bp._STAGES.items) == 1
+    assert _same(out, _direct(K, y, vg))
