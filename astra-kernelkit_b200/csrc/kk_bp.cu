@@ -705,6 +705,27 @@ extern "C" int32_t kk_bp_launches(int64_t n_angles) {
     return n_angles < 1 ? 0 : (int32_t)((n_angles + BP_LAUNCH_ANGLES - 1) / BP_LAUNCH_ANGLES);
 }
 
+// While any thread records a stream into a graph (in CUDA's global mode,
+// torch's default), calls that allocate, free or look at events fail for
+// every thread and end that recording. Textures are made and given back
+// whenever their owners come and go, on streams that have nothing to do with
+// it: within this scope the calling thread is let through.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+extern "C" int kk_exchange_capture_mode(int32_t* mode) {
+    if (!mode || *mode < cudaStreamCaptureModeGlobal || *mode > cudaStreamCaptureModeRelaxed)
+        return kk_fail(KK_ERR_INVALID_ARGUMENT, "kk_exchange_capture_mode: bad mode");
+    cudaStreamCaptureMode m = (cudaStreamCaptureMode)*mode;
+    const cudaError_t e = cudaThreadExchangeStreamCaptureMode(&m);
+    if (e != cudaSuccess) return kk_fail(KK_ERR_CUDA, "kk_exchange_capture_mode: %s", cudaGetErrorString(e));
+    *mode = (int32_t)m;
+    return KK_OK;
+}
+
 extern "C" int kk_layered_create(int64_t layers, int64_t height, int64_t width, int32_t dtype, kk_layered** out) {
     if (!out) return kk_fail(KK_ERR_INVALID_ARGUMENT, "kk_layered_create: out is NULL");
     *out = nullptr;
@@ -722,6 +743,7 @@ extern "C" int kk_layered_create(int64_t layers, int64_t height, int64_t width, 
     t->height = height;
     t->width = width;
     t->dtype = dtype;
+    const RelaxedCapture relaxed;
     cudaError_t e = cudaMalloc3DArray(&t->array, &ch, make_cudaExtent(width, height, layers),
                                       cudaArrayLayered | cudaArraySurfaceLoadStore);
     if (e != cudaSuccess) {
@@ -750,6 +772,7 @@ extern "C" int kk_layered_create(int64_t layers, int64_t height, int64_t width, 
 
 extern "C" int kk_layered_destroy(kk_layered* t) {
     if (!t) return KK_OK;
+    const RelaxedCapture relaxed;
     if (t->surf) cudaDestroySurfaceObject(t->surf);
     cudaDestroyTextureObject(t->tex);
     cudaFreeArray(t->array);
@@ -842,6 +865,7 @@ extern "C" int kk_gather_create(int64_t layers, int64_t height, int64_t width, k
     t->height = height;
     t->width = width;
     t->tiles_x = (int)nx;
+    const RelaxedCapture relaxed;
     e = cudaMallocArray(&t->array, &ch, (size_t)(nx * (width + 2) + 2), (size_t)(ny * (height + 2) + 2),
                         cudaArrayTextureGather | cudaArraySurfaceLoadStore);
     if (e != cudaSuccess) {
@@ -867,6 +891,7 @@ extern "C" int kk_gather_create(int64_t layers, int64_t height, int64_t width, k
 
 extern "C" int kk_gather_destroy(kk_gather* t) {
     if (!t) return KK_OK;
+    const RelaxedCapture relaxed;
     if (t->surf) cudaDestroySurfaceObject(t->surf);
     if (t->tex) cudaDestroyTextureObject(t->tex);
     cudaFreeArray(t->array);

@@ -6,6 +6,7 @@ projection call raises.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from typing import Sequence
@@ -124,7 +125,7 @@ EXPORTS = ("kk_cone_fp_ex", "kk_fp_launches_ex", "kk_wait_timeouts",
            "kk_cone_bp_update", "kk_layered_create", "kk_layered_copy",
            "kk_layered_destroy", "kk_layered_fill", "kk_cone_bp_layered",
            "kk_cone_bp_layered_ex", "kk_gather_create", "kk_gather_destroy",
-           "kk_gather_fill", "kk_cone_bp_gather",
+           "kk_gather_fill", "kk_cone_bp_gather", "kk_exchange_capture_mode",
            "kk_cone_bp_layered_update", "kk_preweight", "kk_filter_rows",
            "kk_reciprocal", "kk_sirt_update", "kk_fp_set_span",
            "kk_fp_launches", "kk_last_error",
@@ -183,6 +184,7 @@ def load():
     L.kk_layered_fill.argtypes = [vp, P(kk_projections), i64, i64, vp]
     L.kk_cone_bp_layered_ex.argtypes = [vp, i64, P(kk_volume), vp, f32, i32,
                                         i32, vp, vp]
+    L.kk_exchange_capture_mode.argtypes = [P(i32)]
     L.kk_gather_create.argtypes = [i64, i64, i64, P(vp)]
     L.kk_gather_destroy.argtypes = [vp]
     L.kk_gather_fill.argtypes = [vp, P(kk_projections), i64, i64, vp]
@@ -258,6 +260,19 @@ def current_stream() -> ctypes.c_void_p:
         return ctypes.c_void_p(t._C._cuda_getCurrentRawStream(
             t._C._cuda_getDevice()))
     return ctypes.c_void_p(t.cuda.current_stream().cuda_stream)
+
+
+@contextlib.contextmanager
+def relaxed_capture():
+    """Scope in which this thread may wait for events (and allocate and
+    free) while a stream is being recorded into a CUDA graph, without ending
+    that recording; the streams it uses must not be the recorded ones."""
+    mode = ctypes.c_int32(2)
+    check(load().kk_exchange_capture_mode(ctypes.byref(mode)))
+    try:
+        yield
+    finally:
+        check(load().kk_exchange_capture_mode(ctypes.byref(mode)))
 
 
 def volume_desc(t, volume_axes: Sequence[int] = (0, 1, 2)) -> kk_volume:

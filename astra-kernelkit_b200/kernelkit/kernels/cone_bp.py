@@ -54,6 +54,11 @@ class _StagePool:
             if not list(self.users):  # len() still counts the one going
                 self.items.clear()
 
+    @staticmethod
+    def _idle(item):
+        with _native.relaxed_capture():
+            return item["used"].query()
+
     def take(self, shape, gather=False):
         """A texture (``gather``: one for exact weights) of at least
         ``shape[0]`` layers, with the current stream made to wait for its
@@ -65,7 +70,7 @@ class _StagePool:
                and isinstance(i["texture"], _native.Gather) == gather
                and i["texture"].shape[1:] == shape[1:]
                and i["texture"].shape[0] >= shape[0]]
-        ready = [i for i in fit if i["stream"] == stream or i["used"].query()]
+        ready = [i for i in fit if i["stream"] == stream or self._idle(i)]
         if ready:
             item = ready[-1]
         elif len(fit) == self.LIMIT:
@@ -96,8 +101,9 @@ def release_staging_textures() -> None:
     """Free the textures that backprojections of lists, other layouts and
     exact weights stage their projections in (waits for their last use)."""
     with _STAGES.lock:
-        for item in _STAGES.items:
-            item["used"].synchronize()
+        with _native.relaxed_capture():
+            for item in _STAGES.items:
+                item["used"].synchronize()
         _STAGES.items.clear()
 
 

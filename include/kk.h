@@ -336,6 +336,12 @@ KK_API int kk_layered_copy(kk_layered* tex, const kk_projections* src,
                            void* stream);
 KK_API int kk_layered_destroy(kk_layered* tex);
 
+/* Exchange the calling thread's stream-capture mode with *mode (0 global, 1
+ * thread-local, 2 relaxed: cudaThreadExchangeStreamCaptureMode). The calls
+ * that create and destroy textures are relaxed by themselves, so they may
+ * come while another stream is recorded into a graph. */
+KK_API int kk_exchange_capture_mode(int32_t* mode);
+
 /* Fill layers [0, count) from projections [first, first + count) of any
  * layout (strides or a pointer table; float32), for callers that stage a
  * scan through a texture of fewer layers. */

@@ -1,7 +1,9 @@
 """Staging textures of the backprojection: the tiles that exact weights
-gather from, no memory for a texture."""
+gather from, no memory for a texture, a graph being recorded on another
+stream."""
 from __future__ import annotations
 
+import gc
 import math
 
 import numpy as np
@@ -10,6 +12,7 @@ import torch
 
 import kernelkit as kk
 from kernelkit import _native
+from kernelkit.algo import capture_graph
 from kernelkit.kernels import VoxelDrivenConeBP, cone_bp
 from kernelkit.kernels.cone_fp import interp_code
 
@@ -126,3 +129,55 @@ def test_frames_too_large_for_gathers(n, monkeypatch):
     K(y, out, vg, additive=False)
     assert len(cone_bp._STAGES.items) == 1
     assert _same(out, _direct(K, y, vg))
+
+
+def test_other_streams_while_a_graph_is_recorded():
+    """Textures are made, looked for, evicted and given back on one stream
+    while another one is recorded; the recording goes on."""
+    cases = [_case(9, "exact", rows=20 + r) for r in range(6)]
+    outs = [torch.empty(SHAPE, device="cuda") for _ in cases]
+    x = torch.zeros(1000, device="cuda")
+    side = [torch.cuda.Stream() for _ in range(2)]
+    cone_bp.release_staging_textures()
+    torch.cuda.synchronize()
+
+    def work():
+        x.add_(1.0)
+        for s in side:
+            with torch.cuda.stream(s):
+                for (K, vg, y), o in zip(cases, outs):
+                    K(y, o, vg, additive=False)
+        cone_bp.release_staging_textures()
+        x.mul_(2.0)
+
+    g = capture_graph(work)
+    g.replay()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(x, torch.full_like(x, 6.0))
+    for (K, vg, y), o in zip(cases, outs):
+        assert torch.equal(o, _direct(K, y, vg))
+
+
+def test_textures_collected_while_a_graph_is_recorded():
+    """An operator's texture that the garbage collector frees in the middle
+    of a recording does not end it."""
+    x = torch.zeros(1000, device="cuda")
+    gc.collect()
+
+    class Owner:
+        def __init__(self):
+            self.texture = _native.Layered(64, 64, 64, _native.KK_F32)
+            self.gather = _native.Gather(64, 64, 64)
+            self.cycle = self
+
+    def work():
+        x.add_(1.0)
+        assert gc.collect() > 0
+        x.mul_(2.0)
+
+    Owner()
+    torch.cuda.synchronize()
+    g = capture_graph(work)
+    g.replay()
+    assert torch.equal(x, torch.full_like(x, 2.0))
