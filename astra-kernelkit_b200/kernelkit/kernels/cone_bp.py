@@ -34,8 +34,9 @@ class _StagePool:
     ``LIMIT``, given back when the last kernel is gone (or by
     ``release_staging_textures``). Filling and sampling a texture are
     enqueued under the lock and followed by an event, which its next use on
-    another stream waits for; a texture that is idle or was last used on the
-    current stream is preferred."""
+    another stream waits for, and which is waited for before the texture is
+    freed; a texture that is idle or was last used on the current stream is
+    preferred, and one that is idle where another has to go."""
 
     LIMIT = 4
 
@@ -46,13 +47,23 @@ class _StagePool:
 
     def add(self, kernel):
         with self.lock:
+            if kernel in self.users:
+                return
             self.users.add(kernel)
         weakref.finalize(kernel, self._gone).atexit = False
 
     def _gone(self):
         with self.lock:
             if not list(self.users):  # len() still counts the one going
-                self.items.clear()
+                self.drop(list(self.items))
+
+    def drop(self, items):
+        """Free textures, when the kernels that sample them are done."""
+        with _native.relaxed_capture():
+            for item in items:
+                item["used"].synchronize()
+        for item in items:
+            self.items.remove(item)
 
     @staticmethod
     def _idle(item):
@@ -77,8 +88,9 @@ class _StagePool:
             item = fit[0]
         else:
             if len(self.items) >= self.LIMIT:
-                old = next((i for i in self.items if i not in fit), None)
-                self.items.remove(old or self.items[0])
+                others = [i for i in self.items if i not in fit]
+                self.drop([next((i for i in others if self._idle(i)),
+                                others[0])])
             try:
                 tex = (_native.Gather(*shape) if gather else
                        _native.Layered(*shape, _native.KK_F32))
@@ -101,10 +113,7 @@ def release_staging_textures() -> None:
     """Free the textures that backprojections of lists, other layouts and
     exact weights stage their projections in (waits for their last use)."""
     with _STAGES.lock:
-        with _native.relaxed_capture():
-            for item in _STAGES.items:
-                item["used"].synchronize()
-        _STAGES.items.clear()
+        _STAGES.drop(list(_STAGES.items))
 
 
 class VoxelDrivenConeBP(BaseKernel):
@@ -272,7 +281,6 @@ class VoxelDrivenConeBP(BaseKernel):
     def _staged(self, pdesc, vdesc, vox_vol, additive) -> bool:
         """Backproject through a staging texture, 128 angles at a time;
         False when there is no memory for one."""
-        L = _native.load()
         n = int(pdesc.n_angles)
         shape = (min(_STAGE_ANGLES, n), int(pdesc.rows), int(pdesc.cols))
         gather = self._interp == _native.KK_INTERP_EXACT
@@ -284,23 +292,32 @@ class VoxelDrivenConeBP(BaseKernel):
                 item = _STAGES.take(shape)
             if item is None:
                 return False
-            tex = item["texture"].handle
-            stream = _native.current_stream()
-            for a in range(0, n, _STAGE_ANGLES):
-                m = min(_STAGE_ANGLES, n - a)
-                params = self._params_dev.data_ptr() + a * 12 * 4
-                add = int(bool(additive) or a > 0)
-                if gather:
-                    _native.check(L.kk_gather_fill(tex, pdesc, a, m, stream))
-                    _native.check(L.kk_cone_bp_gather(
-                        tex, m, vdesc, params, float(vox_vol), add, stream))
-                    continue
-                _native.check(L.kk_layered_fill(tex, pdesc, a, m, stream))
-                _native.check(L.kk_cone_bp_layered_ex(
-                    tex, m, vdesc, params, float(vox_vol), self._interp, add,
-                    0, stream))
-            item["used"].record()
+            _STAGES.add(self)  # a copy of a kernel too
+            try:
+                for a in range(0, n, _STAGE_ANGLES):
+                    self._stage(item["texture"].handle, gather, pdesc, a,
+                                min(_STAGE_ANGLES, n - a), vdesc, vox_vol,
+                                additive)
+            finally:  # also of what came before an error
+                item["used"].record()
         return True
+
+    def _stage(self, tex, gather, pdesc, a, m, vdesc, vox_vol, additive):
+        """Fill a staging texture with ``m`` angles from ``a`` on and
+        backproject them."""
+        L = _native.load()
+        stream = _native.current_stream()
+        params = self._params_dev.data_ptr() + a * 12 * 4
+        add = int(bool(additive) or a > 0)
+        if gather:
+            _native.check(L.kk_gather_fill(tex, pdesc, a, m, stream))
+            _native.check(L.kk_cone_bp_gather(tex, m, vdesc, params,
+                                              float(vox_vol), add, stream))
+        else:
+            _native.check(L.kk_layered_fill(tex, pdesc, a, m, stream))
+            _native.check(L.kk_cone_bp_layered_ex(
+                tex, m, vdesc, params, float(vox_vol), self._interp, add, 0,
+                stream))
 
     def __call__(self, textures, volume, volume_geometry: VolumeGeometry,
                  additive: bool = True):

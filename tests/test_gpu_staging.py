@@ -1,8 +1,9 @@
 """Staging textures of the backprojection: the tiles that exact weights
 gather from, no memory for a texture, a graph being recorded on another
-stream."""
+stream, textures that have to go while they are in use, copied kernels."""
 from __future__ import annotations
 
+import copy
 import gc
 import math
 
@@ -181,3 +182,92 @@ def test_textures_collected_while_a_graph_is_recorded():
     g = capture_graph(work)
     g.replay()
     assert torch.equal(x, torch.full_like(x, 2.0))
+
+
+@pytest.mark.parametrize("way", ["evicted", "released", "last kernel gone"])
+def test_textures_in_use_are_waited_for(way, monkeypatch):
+    """No texture is freed before the kernels that sample it are done."""
+    pool = cone_bp._StagePool()
+    monkeypatch.setattr(cone_bp, "_STAGES", pool)
+    ended, busy = [], torch.cuda.Stream()
+    destroy = _native.Layered.__del__
+
+    def log(texture):
+        if id(texture) in events:
+            ended.append(events[id(texture)].query())
+        destroy(texture)
+
+    cases = [_case(3, rows=20 + r) for r in range(pool.LIMIT)]
+    extra = _case(3, rows=40)
+    out = torch.empty(SHAPE, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        for K, vg, y in cases:
+            torch.cuda._sleep(10_000_000)  # some milliseconds
+            K(y.permute(0, 2, 1).contiguous().permute(0, 2, 1), out, vg)
+    events = {id(i["texture"]): i["used"] for i in pool.items}
+    assert len(events) == pool.LIMIT
+    monkeypatch.setattr(_native.Layered, "__del__", log)
+    if way == "evicted":
+        K, vg, y = extra
+        K(y, torch.empty(SHAPE, device="cuda"), vg)
+    elif way == "released":
+        cone_bp.release_staging_textures()
+    else:
+        # (the pool is told of the kernels it has seen in use)
+        del K, y, extra
+        cases.clear()
+        gc.collect()
+        assert pool.items == []
+    assert ended == [True] * (1 if way == "evicted" else pool.LIMIT)
+    monkeypatch.setattr(_native.Layered, "__del__", destroy)
+    torch.cuda.synchronize()
+
+
+def test_copied_kernels_keep_the_textures(monkeypatch):
+    pool = cone_bp._StagePool()
+    monkeypatch.setattr(cone_bp, "_STAGES", pool)
+    K, vg, y = _case(7, "exact")
+    out = torch.empty(SHAPE, device="cuda")
+    twin = copy.copy(K)
+    K(y, out, vg, additive=False)
+    twin(y, out, vg, additive=False)
+    del K
+    gc.collect()
+    assert len(pool.items) == 1  # the copy is a user of its own
+    assert torch.equal(out, _direct(twin, y, vg))
+    del twin
+    gc.collect()
+    assert pool.items == []
+
+
+def test_an_error_in_between_is_no_lost_use(monkeypatch):
+    """A call that fails after it has filled the texture still counts as
+    its use."""
+    pool = cone_bp._StagePool()
+    monkeypatch.setattr(cone_bp, "_STAGES", pool)
+    K, vg, y = _case(5)
+    frames = [f.clone() for f in y]
+    out = torch.empty(SHAPE, device="cuda")
+    K(frames, out, vg)
+    item, = pool.items
+    torch.cuda.synchronize()
+
+    class Library:
+        def __getattr__(self, name):
+            if name == "kk_cone_bp_layered_ex":
+                return lambda *args: _native.KK_ERR_UNSUPPORTED
+            return getattr(_native.load(), name)
+
+    class Native:
+        load = Library
+
+        def __getattr__(self, name):
+            return getattr(_native, name)
+
+    monkeypatch.setattr(cone_bp, "_native", Native())
+    torch.cuda._sleep(100_000_000)
+    with pytest.raises(NotImplementedError):
+        K(frames, out, vg)
+    assert not item["used"].query()
+    torch.cuda.synchronize()
