@@ -333,17 +333,32 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+#: functions that give back textures kept for later calls, called when there
+#: is no memory for a new one
+RECLAIM = []
+
+
+def _create(create, *args):
+    """The handle that ``create(*args, &handle)`` makes; with no memory for
+    it, tried again without the textures that are kept for later calls."""
+    h = ctypes.c_void_p()
+    try:
+        check(create(*args, ctypes.byref(h)))
+    except KernelKitError:
+        for give_back in RECLAIM:
+            give_back()
+        check(create(*args, ctypes.byref(h)))
+    return h
+
+
 class Layered:
     """Owner of a ``kk_layered`` texture (destroyed with the object)."""
 
     def __init__(self, layers, height, width, dtype):
         self.shape = (int(layers), int(height), int(width))
         self.dtype = int(dtype)
-        h = ctypes.c_void_p()
-        check(load().kk_layered_create(self.shape[0], self.shape[1],
-                                       self.shape[2], self.dtype,
-                                       ctypes.byref(h)))
-        self.handle = h
+        self.handle = _create(load().kk_layered_create, *self.shape,
+                              self.dtype)
 
     def copy_from(self, t):
         """Copy a (layers, height, width) CUDA tensor on the current
@@ -367,9 +382,7 @@ class Gather:
 
     def __init__(self, layers, height, width):
         self.shape = (int(layers), int(height), int(width))
-        h = ctypes.c_void_p()
-        check(load().kk_gather_create(*self.shape, ctypes.byref(h)))
-        self.handle = h
+        self.handle = _create(load().kk_gather_create, *self.shape)
 
     def __del__(self):
         h = getattr(self, "handle", None)

@@ -31,8 +31,8 @@ _STAGE_ANGLES = 128
 
 class _StagePool:
     """Textures that stage projections, shared by all kernels: at most
-    ``LIMIT``, given back when the last kernel is gone (or by
-    ``release_staging_textures``). Filling and sampling a texture are
+    ``LIMIT``, given back when the last kernel is gone, when there is no
+    memory for another texture or by ``release_staging_textures``. Filling and sampling a texture are
     enqueued under the lock and followed by an event, which its next use on
     another stream waits for, and which is waited for before the texture is
     freed; a texture that is idle or was last used on the current stream is
@@ -114,6 +114,9 @@ def release_staging_textures() -> None:
     exact weights stage their projections in (waits for their last use)."""
     with _STAGES.lock:
         _STAGES.drop(list(_STAGES.items))
+
+
+_native.RECLAIM.append(release_staging_textures)
 
 
 class VoxelDrivenConeBP(BaseKernel):

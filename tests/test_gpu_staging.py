@@ -271,3 +271,20 @@ def test_an_error_in_between_is_no_lost_use(monkeypatch):
         K(frames, out, vg)
     assert not item["used"].query()
     torch.cuda.synchronize()
+
+
+def test_given_back_when_there_is_no_memory_for_another_texture():
+    K, vg, y = _case(5, "exact")
+    out = torch.empty(SHAPE, device="cuda")
+    K(y, out, vg)
+    assert cone_bp._STAGES.items
+    made = []
+
+    def create(handle):  # fails as long as the pool keeps something
+        made.append(len(cone_bp._STAGES.items))
+        return _native.KK_ERR_CUDA if made[-1] else _native.KK_OK
+
+    _native._create(create)
+    assert len(made) == 2 and made[-1] == 0
+    K(y, out, vg, additive=False)
+    assert torch.equal(out, _direct(K, y, vg))
