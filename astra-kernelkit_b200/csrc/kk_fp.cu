@@ -1294,10 +1294,9 @@ static int check_residual_aliasing(const kk_projections* out, const kk_fp_residu
     return KK_OK;
 }
 
-extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, const kk_fp_angle* angles,
-                             const float* out_scale, const kk_fp_options* opts, void* stream) {
+static int cone_fp(const kk_volume* vol, const kk_projections* proj, const kk_fp_angle* angles, const float* out_scale,
+                   const kk_fp_options* opts, void* stream) {
     const char* who = "kk_cone_fp_ex";
-    if (!opts) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: options are NULL", who);
     if (opts->span < -1) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: span %d", who, opts->span);
     FpArgs L;
     int rc = fill_fp_args(L, vol, proj, angles, out_scale, opts->interp, opts->slab, who);
@@ -1341,6 +1340,22 @@ extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, c
         return launch_fp<FP_RESIDUAL>(L, vdt, proj->dtype, tex8, (cudaStream_t)stream, lo);
     }
     return launch_fp<FP_STORE>(L, vdt, proj->dtype, tex8, (cudaStream_t)stream, lo);
+}
+
+extern "C" int kk_cone_fp_ex(const kk_volume* vol, const kk_projections* proj, const kk_fp_angle* angles,
+                             const float* out_scale, const kk_fp_options* opts, void* stream) {
+    if (!opts) return kk_fail(KK_ERR_INVALID_ARGUMENT, "kk_cone_fp_ex: options are NULL");
+    const int rc = cone_fp(vol, proj, angles, out_scale, opts, stream);
+    // also after an error, which may have come behind a launch
+    cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+    if ((opts->flags & KK_FP_OPT_DONE) && opts->done &&
+        cudaStreamIsCapturing((cudaStream_t)stream, &recording) == cudaSuccess &&
+        recording == cudaStreamCaptureStatusNone) {
+        const cudaError_t e = cudaEventRecord((cudaEvent_t)opts->done, (cudaStream_t)stream);
+        if (e != cudaSuccess && rc == KK_OK)
+            return kk_fail(KK_ERR_CUDA, "kk_cone_fp_ex: event: %s", cudaGetErrorString(e));
+    }
+    return rc;
 }
 
 extern "C" int kk_fp_set_span(int32_t slices) {

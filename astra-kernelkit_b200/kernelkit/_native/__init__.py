@@ -51,7 +51,7 @@ class kk_fp_options(ctypes.Structure):
                 ("flags", ctypes.c_int32), ("vtex", ctypes.c_void_p),
                 ("residual", ctypes.c_void_p), ("sums", ctypes.c_void_p),
                 ("sums_elems", ctypes.c_int64), ("padded", ctypes.c_void_p),
-                ("padded_elems", ctypes.c_int64)]
+                ("padded_elems", ctypes.c_int64), ("done", ctypes.c_void_p)]
 
 
 #: kk_fp_options.flags: shared-memory tiles staged by the tensor-copy
@@ -61,6 +61,8 @@ KK_FP_OPT_TILES = 1
 KK_FP_OPT_GENERAL = 2
 #: the padded copy of a 16-bit volume is float32
 KK_FP_OPT_PADDED_FLOAT = 4
+#: the event ``done`` is recorded at the end of the call
+KK_FP_OPT_DONE = 8
 
 
 class kk_bp_update(ctypes.Structure):

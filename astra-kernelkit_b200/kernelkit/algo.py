@@ -377,6 +377,7 @@ class SIRT:
         shape = tuple(int(s) for s in volume_geometry.shape)
         self.fp = RayDrivenConeFP(interpolation=interpolation)
         self.fp.half_texture = half
+        self.fp.single_owner = True
         self.fp.compile()
         self.fp.set_params(self.fp.geoms2params(projection_geometry,
                                                 volume_geometry))

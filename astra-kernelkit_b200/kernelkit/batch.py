@@ -153,6 +153,8 @@ class BatchedSIRT:
             ptrs = (ctypes.c_void_p * m)(*[p for p, _ in pads])
             elems = (ctypes.c_int64 * m)(*[e for _, e in pads])
             fo = _native.kk_fp_batch_options(ptrs, elems)
+            # keep the buffers alive with the options
+            fo._pads = [s.fp._workspaces() for s in self.solvers[g:g + m]]
             ba = (_native.kk_bp_problem * m)(*self._bp[g:g + m])
             opts = None
             if self.persistent:

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import copy
 import ctypes
+import threading
 from typing import Sequence
 
 import numpy as np
@@ -94,6 +95,69 @@ def _sequence(projection_geometry) -> ProjectionGeometrySequence:
     return ProjectionGeometrySequence.fromList(projection_geometry)
 
 
+class _Turns:
+    """Turns at the workspaces of a projector (volume texture, padded copy,
+    running sums, the adjoint's ray set-ups), which every call refills: one
+    call is enqueued at a time, and one on another stream than the last
+    waits for it there, as does the memory of the buffers when it is freed.
+    Calls recorded into a CUDA graph only take the lock: their replays are
+    ordered by whoever launches them."""
+
+    def __init__(self):
+        self._lock = threading.RLock()
+        self._last = self._event = None
+        #: handle of the event that ends the current call (None: none does)
+        self.done = None
+
+    def __deepcopy__(self, memo):
+        return _Turns()
+
+    def __reduce__(self):
+        return _Turns, ()
+
+    def next(self, buffers):
+        """The context of one call; ``buffers()`` are the workspaces. The
+        call records ``done``."""
+        self._lock.acquire()
+        try:
+            c = _arrays.torch()._C
+            device = c._cuda_getDevice()
+            key = device, c._cuda_getCurrentRawStream(device)
+            if key != self._last or self.done is None:
+                self._switch(key, buffers)
+        except BaseException:
+            self._lock.release()
+            raise
+        return self
+
+    def _switch(self, key, buffers):
+        t = _arrays.torch()
+        if t.cuda.is_current_stream_capturing():
+            self.done = None
+            return
+        stream = t.cuda.current_stream()
+        if self._last is not None and key != self._last:
+            stream.wait_event(self._event)
+            for b in buffers():
+                b.record_stream(stream)
+        if self._last is None or self._last[0] != key[0]:
+            self._event = t.cuda.Event()
+            self._event.record(stream)  # which creates it
+        self._last, self.done = key, self._event.cuda_event
+
+    def record(self):
+        """``done``, where no library call takes it."""
+        t = _arrays.torch()
+        if self.done is not None and not t.cuda.is_current_stream_capturing():
+            self._event.record()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self._lock.release()
+
+
 class RayDrivenConeFP(BaseKernel):
     """Ray-driven (Joseph) cone-beam forward projection.
 
@@ -135,6 +199,9 @@ class RayDrivenConeFP(BaseKernel):
     #: in pairs, the slabs that cross the volume's boundary without
     #: per-texel tests; same results, with exact weights up to rounding)
     padded_copy = True
+    #: the owner of this projector makes no two calls at a time, in CUDA
+    #: graphs either, and keeps it as long as those
+    single_owner = False
 
     def __init__(self, pixels_per_block: tuple = None,
                  slices_per_block: int = None,
@@ -172,6 +239,7 @@ class RayDrivenConeFP(BaseKernel):
         self._n_params = 0
         self._general = False
         self._axes_known = False
+        self._turns = _Turns()
 
     @property
     def volume_axes(self) -> tuple:
@@ -342,6 +410,12 @@ class RayDrivenConeFP(BaseKernel):
         return lay
 
     # -- launch -------------------------------------------------------------
+    def _workspaces(self):
+        """The device buffers that calls keep for the next one."""
+        held = (getattr(self, name, None) for name in
+                ("_pad_buf", "_sums_buf", "_half_stage", "_adj_work"))
+        return [b for b in held if b is not None]
+
     def _output(self, projections, projection_geometry, projections_pitch):
         """(descriptor, keep-alive objects) for the projections argument."""
         t = _arrays.torch()
@@ -417,8 +491,9 @@ class RayDrivenConeFP(BaseKernel):
                 f"Projections of {pdesc.rows}x{pdesc.cols} pixels do not "
                 f"match the detector {int(det.rows[0])}x{int(det.cols[0])}.")
         osc = self._output_scale_array(volume_geometry.voxel_size)
-        lay = self._volume_texture(vol, vdesc)
-        self._launch(vdesc, pdesc, osc, lay, None, additive)
+        with self._turns.next(self._workspaces):
+            lay = self._volume_texture(vol, vdesc)
+            self._launch(vdesc, pdesc, osc, lay, None, additive)
         del keep
 
     def _sums(self, pdesc):
@@ -448,10 +523,17 @@ class RayDrivenConeFP(BaseKernel):
 
     def _padded(self, vdesc):
         """(pointer, elements) of the zero-padded volume copy's buffer,
-        allocated once per projector, device, volume shape and type."""
+        allocated once per projector, device, volume shape and type. Exact
+        weights recorded into a CUDA graph have none, like their
+        backprojection: nothing would order the graph's use of the buffer
+        against that of other calls (with texture weights the graph shares
+        the volume texture with them in any case)."""
         if not self.padded_copy:
             return None, 0
         t = _arrays.torch()
+        if (self._interp == _native.KK_INTERP_EXACT and not self.single_owner
+                and t.cuda.is_current_stream_capturing()):
+            return None, 0
         dt = {_native.KK_F32: t.float32, _native.KK_BF16: t.bfloat16,
               _native.KK_F16: t.float16}[int(vdesc.dtype)]
         if self._pads_float(vdesc):
@@ -495,6 +577,8 @@ class RayDrivenConeFP(BaseKernel):
 
     def _launch(self, vdesc, pdesc, osc, lay, residual, additive):
         o = self._options(lay, residual, additive, pdesc, vdesc)
+        o.flags |= _native.KK_FP_OPT_DONE
+        o.done = self._turns.done
         _native.check(_native.load().kk_cone_fp_ex(
             vdesc, pdesc, self._params_dev.data_ptr(), osc.ctypes.data, o,
             _native.current_stream()))
@@ -538,15 +622,18 @@ class RayDrivenConeFP(BaseKernel):
         chunk = max(1, min(self._n_params,
                            int(self.adjoint_work_bytes) // (20 * per)))
         need = 5 * chunk * per
-        work = getattr(self, "_adj_work", None)
-        if work is None or work.numel() < need or work.device != vol.device:
-            work = t.empty(need, dtype=t.float32, device=vol.device)
-            self._adj_work = work
         osc = self._output_scale_array(volume_geometry.voxel_size)
-        _native.check(_native.load().kk_cone_fp_adjoint(
-            pdesc, vdesc, self._params_dev.data_ptr(), osc.ctypes.data,
-            self._interp, self.slices_per_block, int(bool(additive)),
-            work.data_ptr(), work.numel(), _native.current_stream()))
+        with self._turns.next(self._workspaces):
+            work = getattr(self, "_adj_work", None)
+            if (work is None or work.numel() < need
+                    or work.device != vol.device):
+                work = t.empty(need, dtype=t.float32, device=vol.device)
+                self._adj_work = work
+            _native.check(_native.load().kk_cone_fp_adjoint(
+                pdesc, vdesc, self._params_dev.data_ptr(), osc.ctypes.data,
+                self._interp, self.slices_per_block, int(bool(additive)),
+                work.data_ptr(), work.numel(), _native.current_stream()))
+            self._turns.record()
         del keep
 
     def residual(self, volume, projection_geometry,
@@ -565,8 +652,9 @@ class RayDrivenConeFP(BaseKernel):
                 raise ValueError(f"`{name}` must have the layout of `out`.")
         res = _native.kk_fp_residual(measured.data_ptr(), weight.data_ptr())
         osc = self._output_scale_array(volume_geometry.voxel_size)
-        lay = self._volume_texture(volume, vdesc)
-        self._launch(vdesc, pdesc, osc, lay, res, False)
+        with self._turns.next(self._workspaces):
+            lay = self._volume_texture(volume, vdesc)
+            self._launch(vdesc, pdesc, osc, lay, res, False)
 
 
 #: span of projectors whose ``slices_per_launch`` is None

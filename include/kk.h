@@ -203,6 +203,11 @@ typedef struct {
                              texture-compatible weights; exact weights may
                              round differently. */
     int64_t padded_elems; /* elements of padded */
+    void* done;           /* with KK_FP_OPT_DONE: NULL, or a CUDA event that
+                             is recorded at the end of the call (not while
+                             the stream is recorded into a graph), for
+                             callers that share sums, padded or vtex between
+                             streams */
 } kk_fp_options;
 
 /* kk_fp_options.flags: rays traced on the CUDA cores sample shared-memory
@@ -221,6 +226,8 @@ typedef struct {
  * the copy converts a 16-bit volume (same results: every sample converts
  * its texels otherwise). */
 #define KK_FP_OPT_PADDED_FLOAT 4
+/* kk_fp_options.flags: the struct has the field `done`. */
+#define KK_FP_OPT_DONE 8
 
 /* The forward projection with every option per call: kk_cone_fp,
  * kk_cone_fp_residual and kk_cone_fp_layered are this entry point with
