@@ -1,5 +1,7 @@
 // Cone-beam backprojection (voxel-driven) for sm_100a: kernel, layered
 // projection textures and the kk_cone_bp* entry points of include/kk.h.
+#include <limits.h>
+
 #include <algorithm>
 #include <mutex>
 
@@ -818,7 +820,10 @@ extern "C" int kk_layered_fill(kk_layered* t, const kk_projections* src, int64_t
         return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: projections [%lld, %lld) do not fit the texture", who,
                        (long long)first, (long long)(first + count));
     const cudaStream_t s = (cudaStream_t)stream;
-    if (!src->table && src->stride[2] == 1 && src->stride[0] == src->rows * src->stride[1]) {
+    // the copy engine's kernel takes rows of one pitch that do not overlap
+    // (arrays may: sliding windows over one long row)
+    if (!src->table && src->stride[2] == 1 && src->stride[0] == src->rows * src->stride[1] &&
+        src->stride[1] >= src->cols && src->stride[1] <= INT_MAX / 4) {
         cudaMemcpy3DParms cp = {};
         cp.srcPtr = make_cudaPitchedPtr((float*)src->data + first * src->stride[0], (size_t)src->stride[1] * 4,
                                         (size_t)src->cols, (size_t)src->rows);

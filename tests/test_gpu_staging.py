@@ -288,3 +288,18 @@ def test_given_back_when_there_is_no_memory_for_another_texture():
     assert len(made) == 2 and made[-1] == 0
     K(y, out, vg, additive=False)
     assert torch.equal(out, _direct(K, y, vg))
+
+
+@pytest.mark.parametrize("interp", ["texture", "exact"])
+@pytest.mark.parametrize("strides", [(41, 1, 1), (41 * 3, 3, 1), (7, 2, 1),
+                                     (2, 1, 3)])
+def test_overlapping_frames(strides, interp):
+    """Sliding windows over one row, whose rows overlap, are projections
+    like any others."""
+    K, vg, y = _case(9, interp)
+    y = y.reshape(-1).as_strided((9, 41, 45), strides)
+    K._layered_source = lambda textures: None
+    out = torch.empty(SHAPE, device="cuda")
+    K(y, out, vg, additive=False)
+    ref = _direct(K, y, vg)
+    assert (out - ref).norm() <= 1e-6 * ref.norm()
