@@ -38,6 +38,10 @@ struct FptArgs {
     const kk_fp_angle* angles;
     float os[9];
     int slab;
+    // by how far slice coordinates may be off the straight line, e per world
+    // axis: half a texel and e; the least D2 step of a walked column, 2 e or
+    // more
+    float margin[3], min_step[3];
     int rec0, nrec;  // records of this chunk
     int accumulate;  // add to the volume (later chunks, or additive)
     float4* ray_ab;  // per * nrec entries, laid out per record (RayRecord)
@@ -249,12 +253,13 @@ __device__ float gather_record(const FptArgs& L, int k, int w0, int w1, int w2) 
     const int rule = 2 - rA;
     const bool a_fast = r1 < r2;
     const float t = (float)s - 0.5f * (float)nS + 0.5f;
-    int c0, c1, rlo, rhi;
-    footprint_box(L, P, A, D1, t, (float)jv - 0.5f - half1, (float)jv + 1.5f - half1, (float)kv - 0.5f - half2,
-                  (float)kv + 1.5f - half2, c0, c1, rlo, rhi);
     const int off = (s / L.slab) * L.slab;
     const float t1 = __fadd_rn(__fsub_rn((float)off, 0.5f * (float)nS), 0.5f);
     const int nst = s - off;
+    const float e1 = D1 == 0 ? L.margin[0] : L.margin[1], e2 = D2 == 0 ? L.margin[0] : L.margin[2];
+    int c0, c1, rlo, rhi;
+    footprint_box(L, P, A, D1, t, (float)jv - e1 - half1, (float)(jv + 1) + e1 - half1, (float)kv - e2 - half2,
+                  (float)(kv + 1) + e2 - half2, c0, c1, rlo, rhi);
     const RayRecord O = ray_record(L, k);
     float acc = 0.f;
     for (int c = c0; c <= c1; ++c) {
@@ -329,8 +334,9 @@ __global__ void __launch_bounds__(FPT_TILE_2* FPT_TILE_1) fpt_gather_kernel(cons
 //
 // Lane 0 is the row before the first owned one: it only hands its second
 // row's sums on. A column whose D2 step per detector row is below 1/16
-// texel or above 1024 texels, or not finite, is handed round the warp and
-// tested ray by ray.
+// texel, or so small that the rounding of its slab's slices might change the
+// order of its rays (FptArgs.min_step), or above 1024 texels, or not finite, is
+// handed round the warp and tested ray by ray.
 //
 // Bound by instruction issue (about 115 warp instructions per 32 (column,
 // texel) pairs, 76 % of the issue slots used) and then by the latency of
@@ -402,8 +408,8 @@ __global__ void __launch_bounds__(32 * WARPS, 36 / WARPS) fpt_column_kernel(cons
             const kk_fp_angle* P = L.angles + L.rec0 + record(g0 + lane);
             if (__ldg(&P->axis) == A && shared_record(P, A, D1)) {
                 int c0, c1, rl, rh;
-                footprint_box(L, P, A, D1, t, (float)j0 - 0.5f - half1, (float)(j0 + FPC_TJ) + 0.5f - half1,
-                              (float)k0 - 0.5f - half2, (float)(k0 + FPC_TK) + 0.5f - half2, c0, c1, rl, rh);
+                footprint_box(L, P, A, D1, t, (float)j0 - L.margin[D1] - half1, (float)(j0 + FPC_TJ) + L.margin[D1] - half1,
+                              (float)k0 - L.margin[D2] - half2, (float)(k0 + FPC_TK) + L.margin[D2] - half2, c0, c1, rl, rh);
                 first = c0;
                 cnt = rh >= rl ? max(c1 - c0 + 1, 0) : 0;
             }
@@ -446,7 +452,7 @@ __global__ void __launch_bounds__(32 * WARPS, 36 / WARPS) fpt_column_kernel(cons
                 z0 = fmaf(e0, t, fmaf(-e0, sA, s2)) + half2;
                 const float z1 = fmaf(e1, t, fmaf(-e1, sA, s2)) + half2;
                 dz = rows > 1 ? (z1 - z0) / (float)(rows - 1) : 1.f;
-                ok = fabsf(dz) >= 0.0625f && fabsf(dz) <= 1024.f && isfinite(z0);
+                ok = fabsf(dz) >= L.min_step[D2] && fabsf(dz) <= 1024.f && isfinite(z0);
                 if (dz < 0.f) z0 = z1;
             }
             const int v1 = sy.i - (j0 - 1);
@@ -465,7 +471,8 @@ __global__ void __launch_bounds__(32 * WARPS, 36 / WARPS) fpt_column_kernel(cons
             auto walk = [&](auto back_tag) {
                 constexpr bool BACK = decltype(back_tag)::value;
                 // start two or less before the first ray whose left texel
-                // may be k0 - 1
+                // may be k0 - 1 (coordinates are off by half a step at most:
+                // the row in hand makes up for it)
                 const bool back = BACK && dz < 0.f;
                 const float pf = floorf(((float)k0 - 0.5f - z0) / fabsf(dz)) - 1.f;
                 int left = in && ok ? rows - (int)fminf(fmaxf(pf, 0.f), (float)rows) : 0;  // rays from here on
@@ -713,6 +720,16 @@ extern "C" int kk_cone_fp_adjoint(const kk_projections* proj, const kk_volume* v
     L.angles = angles;
     for (int k = 0; k < 9; ++k) L.os[k] = out_scale[k];
     L.slab = slab > 0 ? slab : FP_SLAB;
+    // A slice coordinate is the sum of up to nst rounded additions, each off by
+    // at most 2^-24 of the coordinate (rays are at most about 4 texels a slice
+    // steep), and of the few roundings of the slab's start: 7e-4 texel at most
+    // for the default slab on 512 texels, half a texel for 1200 slices on 4000.
+    const int nst = std::min(L.slab, std::max(L.vn[0], std::max(L.vn[1], L.vn[2]))) - 1;
+    for (int k = 0; k < 3; ++k) {
+        const float e = 6e-8f * (float)(nst + 4) * ((float)L.vn[k] + 4.f * (float)nst);
+        L.margin[k] = 0.5f + e;
+        L.min_step[k] = std::max(0.0625f, 2.f * e);
+    }
     const int n = (int)proj->n_angles;
     const int ck = (int)std::min<int64_t>(chunk, n);
     L.ray_ab = (float4*)work;
