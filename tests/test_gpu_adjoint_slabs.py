@@ -1,7 +1,8 @@
 """The exact adjoint where few samples could be lost unseen: slabs of many
 hundred slices on long axes, whose rounded slice coordinates leave the
-straight line by more than the candidate boxes' own margin. Checked by
-<A x, y> = <x, A^T y>."""
+straight line by more than the candidate boxes' own margin, and volumes with
+enough tiles for the four-warp column kernel, with so few rays that every
+sample counts. Checked by <A x, y> = <x, A^T y>."""
 from __future__ import annotations
 
 import math
@@ -63,3 +64,28 @@ def test_long_slabs(name, tilt, slab, interp):
     pgs = [kk.rotate(g0, yaw=0.0007 * k) for k in range(3)]
     assert _mismatch(pgs, shape, interpolation=interp,
                      slices_per_block=slab) <= 1e-7
+
+
+@pytest.mark.parametrize("interp", ["texture", "exact"])
+@pytest.mark.parametrize("flip", [1.0, -1.0])
+def test_single_rays_of_many_tiles(flip, interp):
+    """300 rays that cross some 60000 samples, 2000 of them at the edges of
+    the tiles' rows and as many at their texels': one lost or doubled moves
+    the identity by about 1 / (300 sqrt(230)), 2e-4. Rounding: sums of up to
+    230 terms, 2^-24 sqrt(230) / sqrt(300), 5e-8; 1e-6 is allowed."""
+    det = kk.Detector(rows=380, cols=260, pixel_height=1.3, pixel_width=1.3)
+    g0 = kk.ProjectionGeometry([-400.0, 0.0, 0.0], [80.0, 0.0, 0.0], det,
+                               v=(0.0, 0.0, flip))
+    pgs = [kk.rotate(g0, yaw=0.1 + 2 * math.pi * k / 5) for k in range(5)]
+
+    def few(y, g):
+        keep = torch.randperm(y.numel(), generator=g, device="cuda")[:300]
+        out = torch.zeros_like(y)
+        out.view(-1)[keep] = y.view(-1)[keep]
+        return out
+
+    shape = (230, 160, 250)
+    for axis, across in ((0, 1), (1, 0)):  # the four-warp kernel's volumes
+        assert shape[axis] * -(-shape[across] // 31) * -(-shape[2] // 32) \
+            >= 148 * 40
+    assert _mismatch(pgs, shape, few, interpolation=interp) <= 1e-6
