@@ -316,16 +316,15 @@ __global__ void __launch_bounds__(FPT_TILE_2* FPT_TILE_1) fpt_gather_kernel(cons
 // ---------------------------------------------------------------------------
 // Records whose dominant axis is A and whose rows share their D1
 // coordinate. One warp owns FPC_TJ rows (along D1) x FPC_TK texels (along
-// D2) of one slice and keeps their sums in registers, a lane per row, while
-// it walks the records. Work is laid out so that every ray is set up once
+// D2) of one slice and keeps their sums in shared memory, a lane per row,
+// while it walks the records. Work is laid out so that every ray is set up once
 // per warp and nothing is tested per texel:
 //
 //   * the detector columns whose D1 texel pair {i1, i1 + 1} meets the rows
 //     are packed over the lanes, 32 (record, column) pairs at a time across
 //     record boundaries, so the lanes stay busy whatever a record's share;
 //   * down its column a lane's D2 coordinate only grows, so the texels are
-//     visited in order (unrolled: the sums' register is static) and each
-//     takes the lane's next rays, evaluated two at a time in paired FP32,
+//     visited in order and each takes the lane's next rays, evaluated two at a time in paired FP32,
 //     as long as their left texel is the current one. A ray adds to the
 //     current texel and to the carry of the next, for both texel rows: its
 //     four weights, exactly the forward projector's;
@@ -636,13 +635,17 @@ __global__ void __launch_bounds__(32 * WARPS, 36 / WARPS) fpt_column_kernel(cons
 // ===========================================================================
 using namespace kk;
 
+// (slice, tile) pairs of a pass, a block each
+static int64_t column_blocks(const FptArgs& L, int A) {
+    const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
+    return (int64_t)L.vn[A] * ((L.vn[D1] + FPC_TJ - 1) / FPC_TJ) * ((L.vn[D2] + FPC_TK - 1) / FPC_TK);
+}
+
 template <int WARPS>
 static void launch_column_split(const FptArgs& L, int A, bool tex8, cudaStream_t st) {
     const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
     constexpr int threads = 32 * WARPS;
-    // below 2^31 for every volume the library takes (axes below 2^14)
-    const unsigned blocks = (unsigned)((int64_t)L.vn[A] * ((L.vn[D1] + FPC_TJ - 1) / FPC_TJ) *
-                                       ((L.vn[D2] + FPC_TK - 1) / FPC_TK));
+    const unsigned blocks = (unsigned)column_blocks(L, A);
     // rules 0 and 1 with D2 the faster in-slice axis have their own code;
     // the middle + slowest plane (rule 2) and permuted volumes go by weights4
     const bool d2_fast = L.rank[D2] < L.rank[D1];
@@ -663,10 +666,7 @@ static void launch_column_split(const FptArgs& L, int A, bool tex8, cudaStream_t
 // x 100 x 180 2.60 -> 2.43 ms, 64^3 x 96 0.54 -> 0.37 ms; 192 x 192 x 180 x
 // 250, at 54 pairs per SM, 10.62 ms four ways and 10.88 eight ways).
 static void launch_column_pass(const FptArgs& L, int A, bool tex8, cudaStream_t st) {
-    const int D1 = A == 1 ? 0 : 1, D2 = A == 2 ? 0 : 2;
-    const int64_t pairs =
-        (int64_t)L.vn[A] * ((L.vn[D1] + FPC_TJ - 1) / FPC_TJ) * ((L.vn[D2] + FPC_TK - 1) / FPC_TK);
-    if (pairs < (int64_t)kk_sm_count() * 40)
+    if (column_blocks(L, A) < (int64_t)kk_sm_count() * 40)
         launch_column_split<8>(L, A, tex8, st);
     else
         launch_column_split<4>(L, A, tex8, st);
@@ -711,7 +711,9 @@ extern "C" int kk_cone_fp_adjoint(const kk_projections* proj, const kk_volume* v
         if (L.rank[k] == 1) L.m1 = k;
         if (L.rank[k] == 0) L.m2 = k;
     }
-    if ((L.vn[L.m1] + FPT_TILE_1 - 1) / FPT_TILE_1 > MAX_GRID_Y || L.vn[L.m0] > MAX_GRID_Y)
+    // (volumes of 8 TB and more have more tiles than a launch has blocks)
+    if ((L.vn[L.m1] + FPT_TILE_1 - 1) / FPT_TILE_1 > MAX_GRID_Y || L.vn[L.m0] > MAX_GRID_Y ||
+        std::max(column_blocks(L, 0), std::max(column_blocks(L, 1), column_blocks(L, 2))) > INT_MAX)
         return kk_fail(KK_ERR_UNSUPPORTED, "%s: volume too large for one launch", who);
     L.proj = (const float*)proj->data;
     L.table = proj->table;
