@@ -410,7 +410,9 @@ class SIRT:
         # storage type now, and its padded volume copy: they cannot be
         # created during graph capture
         self.fp._volume_texture(self.x, _native.volume_desc(self.x))
-        self.fp._padded(_native.volume_desc(self.x))
+        if self.fp._pads(_native.projections_desc(self.y),
+                         _native.volume_desc(self.x)):
+            self.fp._padded(_native.volume_desc(self.x))
         self.y_tmp = t.empty_like(self.y)
         # the backprojection samples the residual through a layered
         # texture (the reference's filter), refilled every iteration

@@ -197,7 +197,8 @@ class RayDrivenConeFP(BaseKernel):
     #: trace from a copy of the volume with two zero texels around every
     #: axis, made at the start of every call (the CUDA-core rays then sample
     #: in pairs, the slabs that cross the volume's boundary without
-    #: per-texel tests; same results, with exact weights up to rounding)
+    #: per-texel tests; same results, with exact weights, where few rays do
+    #: without, up to rounding)
     padded_copy = True
     #: the owner of this projector makes no two calls at a time, in CUDA
     #: graphs either, and keeps it as long as those
@@ -521,6 +522,20 @@ class RayDrivenConeFP(BaseKernel):
         return (self.half_texture and int(vdesc.dtype) != _native.KK_F32
                 and max(int(n) for n in vdesc.shape) <= 256)
 
+    def _pads(self, pdesc, vdesc) -> bool:
+        """Whether the rays are traced from the padded copy: with exact
+        weights from 8 samples per voxel on. Below, the copy costs more than
+        its paired loads save (512^3, one angle of 128^2 pixels 0.17 ms, 0.66
+        with the copy; 4.5 samples per voxel 1.07 and 1.24, 9 1.93 and 1.90,
+        18 3.19 and 2.64; 256^3 at 4.5 and 9 0.214 and 0.214, 0.328 and
+        0.287)."""
+        if self._interp != _native.KK_INTERP_EXACT:
+            return True
+        shape = [int(n) for n in vdesc.shape]
+        samples = (int(pdesc.n_angles) * int(pdesc.rows) * int(pdesc.cols)
+                   * max(shape))
+        return samples >= 8 * shape[0] * shape[1] * shape[2]
+
     def _padded(self, vdesc):
         """(pointer, elements) of the zero-padded volume copy's buffer,
         allocated once per projector, device, volume shape and type. Exact
@@ -558,7 +573,7 @@ class RayDrivenConeFP(BaseKernel):
         o = _native.kk_fp_options()
         if pdesc is not None:
             o.sums, o.sums_elems = self._sums(pdesc)
-        if vdesc is not None:
+        if vdesc is not None and self._pads(pdesc, vdesc):
             o.padded, o.padded_elems = self._padded(vdesc)
         o.interp = self._interp if lay is None else _native.KK_INTERP_TEX8
         o.slab = self.slices_per_block
