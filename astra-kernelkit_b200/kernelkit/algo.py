@@ -391,10 +391,21 @@ class SIRT:
         self.min_c, self.max_c = min_constraint, max_constraint
         L = _native.load()
         stream = _native.current_stream()
-        # C = 1 / A^T 1 and R = 1 / A 1, formed in float32
+        # the backprojection samples the residual through a layered
+        # texture (the reference's filter), refilled every iteration
+        self.tex = (_native.Layered(*self.y.shape, _native.KK_F16 if half
+                                    else _native.KK_F32)
+                    if interpolation == "texture" and len(self.y) <= 2048
+                    else None)
+        # C = 1 / A^T 1 and R = 1 / A 1, formed in float32 (from a float32
+        # texture: the solver's own, or one that stages the ones)
         C = t.empty(shape, dtype=t.float32, device="cuda")
         ones = t.ones(self.y.shape, dtype=t.float32, device="cuda")
-        self.bp(ones, C, volume_geometry, additive=False)
+        src = ones
+        if self.tex is not None and not half:
+            self.tex.copy_from(ones)
+            src = self.tex
+        self.bp(src, C, volume_geometry, additive=False)
         _native.check(L.kk_reciprocal(C.data_ptr(), C.numel(), stream))
         del ones
         self.C = C if not half else C.to(vdt)
@@ -414,12 +425,6 @@ class SIRT:
                          _native.volume_desc(self.x)):
             self.fp._padded(_native.volume_desc(self.x))
         self.y_tmp = t.empty_like(self.y)
-        # the backprojection samples the residual through a layered
-        # texture (the reference's filter), refilled every iteration
-        self.tex = (_native.Layered(*self.y.shape, _native.KK_F16 if half
-                                    else _native.KK_F32)
-                    if interpolation == "texture" and len(self.y) <= 2048
-                    else None)
         self.bp._work_for(self.x, True)  # allocate before any graph capture
         self._graph = None
 
