@@ -69,7 +69,22 @@ struct FpArgs {
     // of at most 32 rows, with the thread's two rays in two columns;
     // pair_tiles column tiles of 2 FP_COLS (0: no such blocks)
     int pair_tiles, full_blocks;
+    // how near the ends of an axis a slab's first and last sample may come for
+    // the samples between them to be taken as inside (or outside); the same
+    // for all axes, as an operand that takes the kernels no register
+    float margin;
 };
+
+// How far a slice coordinate may be off the straight line along an axis of n
+// texels: it is the sum of up to nst rounded additions, each off by at most
+// 2^-24 of the coordinate (rays are at most about 4 texels a slice steep), and
+// of the few roundings of the slab's start. 7e-4 texel at most for the default
+// slab on 512 texels, half a texel for 1200 slices on 4000.
+inline float slab_drift(int slab, const int* vn, int axis) {
+    const int longest = vn[0] > vn[1] ? (vn[0] > vn[2] ? vn[0] : vn[2]) : (vn[1] > vn[2] ? vn[1] : vn[2]);
+    const int nst = (slab < longest ? slab : longest) - 1;
+    return 6e-8f * (float)(nst + 4) * ((float)vn[axis] + 4.f * (float)nst);
+}
 
 struct BpArgs {
     const void* proj;

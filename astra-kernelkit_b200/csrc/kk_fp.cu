@@ -119,21 +119,22 @@ __device__ __forceinline__ float fast_sample(float acc, const T* __restrict__ ro
 // Whether the samples of a ray between coordinates c0 and c1 (first and
 // last slice of a slab) can touch a texel of an axis of n texels: the
 // complement of span_class's "every sample reads only border zeros".
-__device__ __forceinline__ bool span_touches(float c0, float c1, int n) {
-    return fmaxf(c0, c1) >= -0.53f && fminf(c0, c1) <= (float)n + 0.53f;
+__device__ __forceinline__ bool span_touches(float c0, float c1, int n, float margin) {
+    return fmaxf(c0, c1) >= -margin && fminf(c0, c1) <= (float)n + margin;
 }
 
 // Slab classification of a ray from its coordinates at the first and last
-// slice of the slab (coordinates move linearly; the float32 increments
-// drift by far less than the margins). 2 = both texels of every sample
-// inside the array, 0 = every sample reads only border zeros, 1 = mixed.
-__device__ __forceinline__ int span_class(float c0, float c1, int n) {
+// slice of the slab (coordinates move linearly, but for the drift of the
+// float32 increments, which FpArgs.margin allows for). 2 = both texels of
+// every sample inside the array, 0 = every sample reads only border zeros,
+// 1 = mixed.
+__device__ __forceinline__ int span_class(float c0, float c1, int n, float margin) {
     const float lo = fminf(c0, c1), hi = fmaxf(c0, c1);
     // texel i = floor(x - 1/2) on the 1/256 grid: i >= 0 iff x >= 0.498,
     // i + 1 <= n - 1 iff x < n - 0.502; both out iff x < -0.502 or
     // x >= n + 0.498
-    if (lo >= 0.53f && hi <= (float)n - 0.53f) return 2;
-    if (hi < -0.53f || lo > (float)n + 0.53f) return 0;
+    if (lo >= margin && hi <= (float)n - margin) return 2;
+    if (hi < -margin || lo > (float)n + margin) return 0;
     return 1;
 }
 
@@ -222,11 +223,11 @@ __device__ __forceinline__ void fp_trace(const FpArgs& L, const kk_fp_angle* P, 
             if (PATH == 3) {
                 // the texture unit handles borders: only slabs that miss
                 // the volume need a test
-                any |= span_touches(yc[k], fmaf(R[k].a1, span, yc[k]), n1) &&
-                       span_touches(zc[k], fmaf(R[k].a2, span, zc[k]), n2);
+                any |= span_touches(yc[k], fmaf(R[k].a1, span, yc[k]), n1, L.margin) &&
+                       span_touches(zc[k], fmaf(R[k].a2, span, zc[k]), n2, L.margin);
             } else if (PATH != 0) {
-                const int cy = span_class(yc[k], fmaf(R[k].a1, span, yc[k]), n1);
-                const int cz = span_class(zc[k], fmaf(R[k].a2, span, zc[k]), n2);
+                const int cy = span_class(yc[k], fmaf(R[k].a1, span, yc[k]), n1, L.margin);
+                const int cz = span_class(zc[k], fmaf(R[k].a2, span, zc[k]), n2, L.margin);
                 const int ck = min(cy, cz);
                 cls = min(cls, ck);
                 any |= ck;
@@ -1006,6 +1007,8 @@ static int fp_span(int nmax, int slab, int setting) {
 // bytes and a 16-byte aligned base. False: the path is not available
 // (the kernel then traces with direct loads).
 static bool brick_prepare(FpBrick& B, const FpArgs& L) {
+    // the windows are a texel wider than the rays: half of it for the drift
+    if (L.margin > 1.f) return false;
     int ax_of_rank[3];
     for (int k = 0; k < 3; ++k) ax_of_rank[L.rank[k]] = k;
     const int r0 = ax_of_rank[0], r1 = ax_of_rank[1], r2 = ax_of_rank[2];
@@ -1257,6 +1260,9 @@ static int fill_fp_args(FpArgs& L, const kk_volume* vol, const kk_projections* p
     L.angles = angles;
     for (int k = 0; k < 9; ++k) L.os[k] = out_scale[k];
     L.slab = slab > 0 ? slab : FP_SLAB;
+    // 0.502 texel (span_class) and the drift: 0.53 up to a drift of 0.028
+    L.margin = 0.53f;
+    for (int k = 0; k < 3; ++k) L.margin = std::max(L.margin, 0.502f + slab_drift(L.slab, L.vn, k));
     if ((int64_t)((L.rows + FP_ROWS_T - 1) / FP_ROWS_T) * L.n_angles * ((L.cols + FP_COLS - 1) / FP_COLS) >=
         0x7fffffffLL)
         return kk_fail(KK_ERR_UNSUPPORTED, "%s: too many projection tiles for one launch", who);

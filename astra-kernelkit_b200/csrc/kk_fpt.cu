@@ -722,13 +722,8 @@ extern "C" int kk_cone_fp_adjoint(const kk_projections* proj, const kk_volume* v
     L.angles = angles;
     for (int k = 0; k < 9; ++k) L.os[k] = out_scale[k];
     L.slab = slab > 0 ? slab : FP_SLAB;
-    // A slice coordinate is the sum of up to nst rounded additions, each off by
-    // at most 2^-24 of the coordinate (rays are at most about 4 texels a slice
-    // steep), and of the few roundings of the slab's start: 7e-4 texel at most
-    // for the default slab on 512 texels, half a texel for 1200 slices on 4000.
-    const int nst = std::min(L.slab, std::max(L.vn[0], std::max(L.vn[1], L.vn[2]))) - 1;
     for (int k = 0; k < 3; ++k) {
-        const float e = 6e-8f * (float)(nst + 4) * ((float)L.vn[k] + 4.f * (float)nst);
+        const float e = slab_drift(L.slab, L.vn, k);
         L.margin[k] = 0.5f + e;
         L.min_step[k] = std::max(0.0625f, 2.f * e);
     }
