@@ -1150,6 +1150,14 @@ static void launch_fp_typed(const FpArgs& base, bool tex8, cudaStream_t s, const
     }
 }
 
+// Storage types a caller may combine. A volume in a float32 copy is launched
+// as a float32 one, which would take more.
+static bool fp_takes(int vdt, int pdt, bool residual) {
+    if (pdt == KK_F32) return vdt == KK_F32 || !residual;
+    if (pdt == KK_F16) return vdt != KK_F32 || !residual;
+    return vdt != KK_F16 && !residual;
+}
+
 template <int EPI>
 static int launch_fp(const FpArgs& L, int vdt, int pdt, bool tex8, cudaStream_t s, const FpLaunch& opt) {
 #define KK_FP_CASE(VD, PD, TV, TP)                                   \
@@ -1309,6 +1317,8 @@ static int cone_fp(const kk_volume* vol, const kk_projections* proj, const kk_fp
     if (rc) return rc;
     const bool tex8 = opts->interp == KK_INTERP_TEX8;
     int vdt = vol->dtype;  // of the volume traced
+    if (!fp_takes(vdt, proj->dtype, opts->residual != nullptr))
+        return kk_fail(KK_ERR_UNSUPPORTED, "%s: dtype combination volume=%d projections=%d", who, vdt, proj->dtype);
     if (opts->vtex) {
         const kk_layered* vtex = opts->vtex;
         if (!tex8) return kk_fail(KK_ERR_INVALID_ARGUMENT, "%s: a volume texture needs texture interpolation", who);
