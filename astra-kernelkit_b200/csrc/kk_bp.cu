@@ -35,11 +35,12 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // bilinear<false>() from a tile of a kk_gather array whose texel (0, 0) is at
 // org - 1: the four texels of the footprint come from one texture gather at
 // its centre, so the lanes of a warp, whose rows differ, do not each fetch
-// their own lines (128 x 128 x 100 x 180 x 150 x 192: 2.34 -> 0.98 ms with
-// the copy into the texture, 0.43 ms for the texture's own weights; the
-// weights' arithmetic now takes the issue slots). Coordinates beyond the
-// tile's two zero rows and columns move onto them, where the sample is zero
-// as well. floor() by rounding down at 2^23: same result, without the
+// their own lines (256^3 x 360 x 384^2: 39.8 -> 10.2 ms with the copy into
+// the texture, 5.4 ms for the texture's own weights). Bound by the gathers'
+// latency (9.3 warps per issue wait for one at 49 % of the warps active; the
+// texture data pipe is 49 % and the issue slots 61 % used). Coordinates beyond
+// the tile's two zero rows and columns move onto them, where the sample is
+// zero as well. floor() by rounding down at 2^23: same result, without the
 // conversion unit.
 __device__ __forceinline__ float gather_exact(cudaTextureObject_t tex, float V, float U, float rows, float cols,
                                               float2 org) {
@@ -76,8 +77,8 @@ __device__ __forceinline__ float surface_exact(cudaSurfaceObject_t surf, float V
 // float32 steps err by less than a tenth of that) keeps the test safe, and
 // a NaN or a corner near the source plane counts as reaching the block.
 //
-// The kernel is bound by the texture unit's fetch rate, with the issue slots
-// close behind (82 % of its cycles). At 512^3 x 720 x 768^2 the cone misses
+// The kernel is bound by the texture unit's fetch rate, without the skipping
+// with the issue slots close behind (82 % of its cycles, 47 % now). At 512^3 x 720 x 768^2 the cone misses
 // 8.9 % of the (block, angle) pairs (6.2 % at 256^3 x 360 x 384^2), whose
 // fetches cost less than others but not nothing. Together with the loop's
 // fewer instructions (rcp_approx and paired accumulation, which alone give

@@ -337,10 +337,10 @@ __global__ void __launch_bounds__(FPT_TILE_2* FPT_TILE_1) fpt_gather_kernel(cons
 // order of its rays (FptArgs.min_step), or above 1024 texels, or not finite, is
 // handed round the warp and tested ray by ray.
 //
-// Bound by instruction issue (about 115 warp instructions per 32 (column,
-// texel) pairs, 76 % of the issue slots used) and then by the latency of
-// the ray loads. 256^3 x 360 x 384^2: 256.5 -> 36.8 ms against a per-texel
-// gather from shared-memory tables, 64^3 x 96 x 96^2: 1.60 -> 0.37 ms. The
+// Bound by instruction issue (80 % of the issue slots used on 384^3 x 128 x
+// 576^2) and then by the latency of the ray loads. 256^3 x 360 x 384^2: 256.5
+// -> 36.6 ms against a per-texel gather from shared-memory tables, 64^3 x 96 x
+// 96^2: 1.60 -> 0.36 ms. The
 // sums live in shared memory, not in registers: a register per texel means
 // unrolling the texel loop, whose code then misses the instruction cache
 // (75 ms).

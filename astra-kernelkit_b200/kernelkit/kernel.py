@@ -116,9 +116,11 @@ class BaseKernel(ABC):
     """Base class of the projection kernels (``kernel.py:166-239``).
 
     Contract kept from the reference (``docs/user_guide/kernels.rst``):
-    ``__call__`` launches work and returns None, performs no device
-    allocation and no device-to-host transfer, so it can be captured in a
-    CUDA graph; ``compile()`` must precede the first call."""
+    ``__call__`` launches work and returns None, without a device-to-host
+    transfer, and can be captured in a CUDA graph: device memory is only
+    allocated for the workspaces and staging textures that a first call
+    makes and later ones find, and captured calls do without those they
+    would share with others; ``compile()`` must precede the first call."""
 
     def __init__(self):
         self._compiled_options = None

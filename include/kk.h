@@ -333,8 +333,8 @@ KK_API int kk_cone_bp_update(const kk_projections* proj, const kk_volume* vol,
 /* A 2D-layered CUDA array of the projections (one layer per angle) with a
  * border-addressed, linearly filtered texture object: the texture the
  * reference's BackProjector samples (projector.py:529-542, kernel.py:
- * 91-96). Created once per scan (this is the only allocating entry
- * point), refilled from device projections with kk_layered_copy, and
+ * 91-96). Created once per scan (this and kk_gather_create are
+ * the only allocating entry points), refilled from device projections with kk_layered_copy, and
  * sampled by kk_cone_bp_layered*, whose interpolation is then the texture
  * unit's own. float32 or float16 texels; at most 2048 layers. */
 KK_API int kk_layered_create(int64_t layers, int64_t height, int64_t width,
