@@ -59,6 +59,8 @@ class _StagePool:
 
     def drop(self, items):
         """Free textures, when the kernels that sample them are done."""
+        if not items:
+            return
         with _native.relaxed_capture():
             for item in items:
                 item["used"].synchronize()

@@ -64,3 +64,16 @@ def test_storage_types_stay_refused(volume, projections, residual, as_float):
                          (ctypes.c_float * 9)(), o, None)
     assert rc == _native.KK_ERR_UNSUPPORTED
     assert b"dtype combination" in L.kk_last_error()
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="no device wanted")
+def test_a_failed_texture_keeps_its_reason():
+    """Giving back the kept textures, of which there are none, does not
+    replace the error that asked for it."""
+    import kernelkit.kernels  # registers what is given back
+
+    assert kernelkit.kernels and _native.RECLAIM
+    with pytest.raises(_native.KernelKitError, match="kk_layered_create"):
+        _native.Layered(1, 1, 1, F32)
+    with pytest.raises(_native.KernelKitError, match="kk_gather_create"):
+        _native.Gather(1, 1, 1)
